@@ -347,7 +347,8 @@ class Assembly:
     def _assemble_plan(self, gc, want_K, K, R):
         """R and K of the plan's rows at the plan displacement gc."""
         P = self.plan
-        R = P.zeros(P.ndof) if R is None else R
+        if R is None:                             # every row is written below, or zeroed first
+            R = torch.empty(P.ndof, dtype=torch.float64, device=P.device)
         if want_K and K is None:
             K = torch.empty(P.nnz, dtype=torch.float64, device=P.device)
         # the first group stores whole rows when it touches every active node;

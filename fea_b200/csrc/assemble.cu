@@ -27,6 +27,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "hexlane.cuh"
 
 namespace fea {
 
@@ -371,10 +372,6 @@ constexpr int HX_LPN = 16;
 __host__ __device__ inline int64_t hx_rslot_base(int64_t nblk) { return (nblk * 9 + 1) & ~(int64_t)1; }
 constexpr int HX_GINC = 32;               // chunk capacity of C3D8 plans (the C3D8 kernels read no chunks)
 
-// corner signs of hex node / Gauss point c (brick.py:15-25, 151-160)
-__device__ __forceinline__ double csx(int c) { return (((c + 1) >> 1) & 1) ? 1.0 : -1.0; }
-__device__ __forceinline__ double csy(int c) { return ((c >> 1) & 1) ? 1.0 : -1.0; }
-__device__ __forceinline__ double csz(int c) { return (c >> 2) ? 1.0 : -1.0; }
 template <bool ER>
 __global__ void __launch_bounds__(HX_TPB, HX_CTAS) k_hex_elem(VolParams P, double* __restrict__ stage,
                                                      double* __restrict__ rslot) {
@@ -754,7 +751,88 @@ __global__ void __launch_bounds__(HX_GW * 32, 8) k_hex_gat(VolParams P, const do
   }
 }
 
-// R-only kernel: one thread per node, sequential over its incidences.
+// ---- C3D8 R only: each element once, then a sum per node --------------------
+// (hexlane.cuh has the scheme.)  Bound by FP64 issue and shared-memory reads:
+// about 420 FP64 operations a Gauss point (20 us of FP64 issue for the 48^3
+// block).  48^3 block: 37.3 us + 10 us for the sum, against 366 us with a
+// thread per node (k_vol_r<8>); five CTAs per SM (8 bytes of spills) 37.3
+// against 38.3 us with four.
+template <bool ER>
+__global__ void __launch_bounds__(HL_TPB, 5) k_hex_force(VolParams P, double* __restrict__ slot) {
+  __shared__ __align__(16) double sv[HL_EPB * HL_EL];
+  const int le = threadIdx.x >> 3, lane = threadIdx.x & 7;
+  const int64_t e = (int64_t)blockIdx.x * HL_EPB + le;
+  const bool act = e < P.ne;
+  double* V = sv + le * HL_EL;
+  unsigned mb = 0;
+  if (act) {
+    const int32_t c = P.conn[e * 8 + lane];
+    const double* xb = P.X + 3 * (int64_t)c;
+    mb = P.mask[c];
+    const int32_t rb = P.rdof[c];
+    double2* o = reinterpret_cast<double2*>(V + 6 * lane);
+    o[0] = make_double2(__ldg(xb), __ldg(xb + 1));
+    o[1] = make_double2(__ldg(xb + 2), node_u(P.gc, rb, mb, 0));
+    o[2] = make_double2(node_u(P.gc, rb, mb, 1), node_u(P.gc, rb, mb, 2));
+  }
+  __syncwarp();
+  const HexLane<double> H(lane);
+  double JJ[2][9];
+  if (act) hex_gradients<double, 2>(H, V, JJ);
+  __syncwarp();                                  // the node data are read: the area takes the matrices
+  if (act) {
+    double iJ[9], F[9], iF[9], M[9], Jm;
+    const double w = inv3(JJ[0], iJ);            // Gauss weight 1
+    const double* Ju = JJ[1];
+#pragma unroll
+    for (int I = 0; I < 3; ++I)
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        F[3 * I + i] = fma(Ju[3 * I], iJ[i], fma(Ju[3 * I + 1], iJ[3 + i], fma(Ju[3 * I + 2], iJ[6 + i], I == i ? 1.0 : 0.0)));
+    const double J = inv3_jm(F, iF, &Jm);
+    double sF2 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) sF2 += F[i] * F[i];
+    const double muJm = P.mu * Jm, c2 = P.kappa * J * (J - 1.0) - P.mu * (Jm * sF2) / 3.0;
+    // M = mu J^-2/3 F + c2 F^-T, r_a = sum_g w M g_a
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) M[3 * j + i] = muJm * F[3 * j + i] + c2 * iF[3 * i + j];
+    hex_put(V, lane, w, M, iJ);
+  }
+  __syncwarp();
+  if (!act) return;
+  double r[3];
+  hex_take(H, V, lane, r);
+  if (!(mb & 7u)) return;                        // no row reads this slot
+  hex_store_slot(slot, e, lane, r);
+  if (ER) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) P.elemR[(int64_t)(3 * lane + j) * P.ne + e] = r[j];
+  }
+}
+
+template <bool ACC>
+__global__ void __launch_bounds__(128) k_hex_force_sum(VolParams P, const double* __restrict__ slot) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= P.n_nodes) return;
+  const unsigned mn = P.mask[n];
+  if (!mn) return;
+  double r[3];
+  hex_sum_slots(slot, P.inc, P.nodeinc[n], P.nodeinc[n + 1], r);
+  double* Rout = P.R + P.rdof[n];
+  int rj = 0;
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    if (mn >> j & 1u) {
+      Rout[rj] = ACC ? Rout[rj] + r[j] : r[j];
+      ++rj;
+    }
+}
+
+// R-only kernel: one thread per node, sequential over its incidences (C3D4,
+// and C3D8 when the caller gives no work buffer).
 template <int NN, bool ACC, bool ER>
 __global__ void __launch_bounds__(128) k_vol_r(VolParams P) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1462,6 +1540,11 @@ extern "C" int64_t fea_assemble_work_len(const fea_group_t* G) {
   return hx_rslot_base(G->nblk) + slots * 4;
 }
 
+extern "C" int64_t fea_force_work_len(const fea_group_t* G) {
+  if (!G || G->kind != FEA_C3D8 || G->ne <= 0) return 0;
+  return G->ne * 8 * HL_SLOT;
+}
+
 extern "C" int fea_assemble_volume(const fea_nodes_t* N, const fea_group_t* G, double mu, double kappa,
                                    const double* gc, double* K, double* R, double* elemR, int32_t accumulate,
                                    double* work, int64_t work_len, cudaStream_t st) {
@@ -1542,6 +1625,15 @@ extern "C" int fea_assemble_volume(const fea_nodes_t* N, const fea_group_t* G, d
   }
   const int grid = grid_for(N->n_nodes, 128);
   if (N->n_nodes == 0) return FEA_OK;
+  if (hex && G->ne > 0 && work && work_len >= fea_force_work_len(G) && ((uintptr_t)work & 15) == 0) {
+    const unsigned eg = (unsigned)((G->ne + HL_EPB - 1) / HL_EPB);
+    if (elemR) k_hex_force<true><<<eg, HL_TPB, 0, st>>>(P, work);
+    else k_hex_force<false><<<eg, HL_TPB, 0, st>>>(P, work);
+    if (accumulate) k_hex_force_sum<true><<<grid, 128, 0, st>>>(P, work);
+    else k_hex_force_sum<false><<<grid, 128, 0, st>>>(P, work);
+    count_launch(2);
+    return (int)cudaGetLastError();
+  }
   if (hex) {
     if (accumulate) elemR ? k_vol_r<8, true, true><<<grid, 128, 0, st>>>(P) : k_vol_r<8, true, false><<<grid, 128, 0, st>>>(P);
     else elemR ? k_vol_r<8, false, true><<<grid, 128, 0, st>>>(P) : k_vol_r<8, false, false><<<grid, 128, 0, st>>>(P);

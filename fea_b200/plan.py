@@ -8,7 +8,9 @@ only launches kernels on the current torch stream.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
+import threading
 
 import numpy as np
 import torch
@@ -17,6 +19,9 @@ from . import _lib as L
 
 KIND = {"C3D4": L.FEA_C3D4, "C3D8": L.FEA_C3D8, "T3": L.FEA_T3, "Q4": L.FEA_Q4}
 NODES_PER = {L.FEA_C3D4: 4, L.FEA_C3D8: 8, L.FEA_T3: 3, L.FEA_Q4: 4}
+
+
+_NO_LOCK = contextlib.nullcontext()
 
 
 def vptr(t):
@@ -149,6 +154,8 @@ class GatherGroup:
                             self.region.data_ptr() if self.region is not None else None, nblk, maxblk,
                             hp.scalar(L.FEA_S_G_HXSTRIDE, index) if uptr.size else 0)
         self.nchunk = int(self.desc.nchunk)
+        # doubles of the element-once kernels' slots (C3D8 elements)
+        self.slot_len = int(L.fea_force_work_len(C.byref(self.desc))) if base == L.G_BASE else 0
 
 
 class DevicePlan:
@@ -190,6 +197,13 @@ class DevicePlan:
                                  self.adjoff.data_ptr(), self.moff.data_ptr())
             self.groups = [GatherGroup(hp, L.G_BASE, i, k, c, self.device) for i, (k, c) in enumerate(gl)]
             self.faces = [GatherGroup(hp, L.F_BASE, i, k, c, self.device) for i, (k, c) in enumerate(fl)]
+            # slots of the element-once kernels (C3D8 residual, adjoint):
+            # laid out here, so that a first call does not wait for them
+            self._slots_len = max([g.slot_len for g in self.groups], default=0)
+            self._slots = (torch.empty(self._slots_len, dtype=torch.float64, device=self.device)
+                           if self._slots_len else None)
+            self._slots_stream = torch.cuda.current_stream().cuda_stream
+            self._slots_lock = threading.Lock()
         self._scratch = None
         self._coo = None
 
@@ -221,16 +235,37 @@ class DevicePlan:
             g._stage = torch.empty(n, dtype=torch.float64, device=self.device)
         return g._stage, n
 
+    def slots(self, n):
+        """(buffer, n, lock): n doubles for the per-element slots of one call,
+        the lock held around its launches; (None, 0, ...) where there is no
+        memory for them (the entry points then take the path that needs
+        none).  Calls on the stream the plan was built on share the buffer
+        laid out with the plan, one call's launches at a time (launches of two
+        host threads do not interleave, and the stream orders them); calls on
+        other streams, or under capture, take a buffer of their own from the
+        caching allocator."""
+        if n <= self._slots_len and not torch.cuda.is_current_stream_capturing() \
+                and torch.cuda.current_stream().cuda_stream == self._slots_stream:
+            return self._slots, n, self._slots_lock
+        try:
+            return torch.empty(n, dtype=torch.float64, device=self.device), n, _NO_LOCK
+        except torch.cuda.OutOfMemoryError:
+            return None, 0, _NO_LOCK
+
     def assemble_volume(self, gi, mu, kappa, gc, K=None, R=None, elemR=None, accumulate=False):
         g = self.groups[gi]
         need(gc, self.ndof, self.device, "gc")
         need(K, self.nnz, self.device, "K")
         need(R, self.ndof, self.device, "R")
         need(elemR, g.nn * 3 * g.ne, self.device, "elemR")
-        w, wn = self.stage(gi) if K is not None else (None, 0)
-        L.check(L.fea_assemble_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
-                                      vptr(K), vptr(R), vptr(elemR), int(bool(accumulate)), vptr(w), int(wn),
-                                      stream()), "fea_assemble_volume")
+        if K is not None or g.slot_len == 0:
+            (w, wn), lock = self.stage(gi) if K is not None else (None, 0), _NO_LOCK
+        else:
+            w, wn, lock = self.slots(g.slot_len)
+        with lock:
+            L.check(L.fea_assemble_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
+                                          vptr(K), vptr(R), vptr(elemR), int(bool(accumulate)), vptr(w), int(wn),
+                                          stream()), "fea_assemble_volume")
 
     def assemble_pressure(self, fi, p, Xinst, gc, K=None, R=None):
         f = self.faces[fi]

@@ -232,8 +232,12 @@ typedef struct {
  * work_dev: fea_assemble_work_len(group) doubles of scratch, 16-byte
  * aligned (C3D8 stages there the upper blocks of every element row, 9
  * doubles each, node by node (nblk blocks), then R_a of every incidence, 4
- * doubles each; C3D4 needs none). */
+ * doubles each; C3D4 needs none).  Without K, a C3D8 group given
+ * fea_force_work_len(group) doubles (16-byte aligned) evaluates each element
+ * once and sums the nodes' contributions there; with less, or NULL, it
+ * evaluates the elements of every node. */
 int64_t fea_assemble_work_len(const fea_group_t* group);
+int64_t fea_force_work_len(const fea_group_t* group);
 int fea_assemble_volume(const fea_nodes_t* nodes, const fea_group_t* group, double mu, double kappa,
                         const double* gc_dev, double* K_dev, double* R_dev, double* elemR_dev,
                         int32_t accumulate, double* work_dev, int64_t work_len, cudaStream_t stream);

@@ -1,0 +1,127 @@
+"""C3D8 kernels that evaluate each element once (slots per element and node,
+then a sum per node) against the general path (every node evaluates its
+elements), which the same entry points take without the slots' buffer.
+
+Meshes: element counts around the 16 of a CTA, one element, constrained
+components, shuffled node numbers, an element that repeats a node.  Both
+paths sum at most 8 elements x 8 Gauss points per entry with relative error
+of a few 1e-15 per term; entries cancel by up to a factor of a hundred in the
+near-incompressible residual: 1e-12 of the largest entry bounds the
+difference."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import fea_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+MESHES = [(1, 1, 1), (5, 3, 1), (4, 2, 2), (17, 1, 1), (3, 4, 5)]
+
+
+def ptr(t):
+    return None if t is None else C.c_void_p(t.data_ptr())
+
+
+def stream():
+    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def hex_plan(dims, shuffle=True, repeat=False, seed=3):
+    """Plan of a jittered block with a clamped node and a partly fixed one,
+    and a displacement; repeat: one element uses a node twice."""
+    from fea_b200 import DevicePlan
+    from fea_b200.meshes import hex_block
+    rng = np.random.default_rng(seed)
+    X, el = hex_block(0, jitter=0.1, seed=seed, dims=dims)
+    N = X.shape[0]
+    if shuffle:
+        perm = rng.permutation(N)
+        inv = np.empty(N, np.int64)
+        inv[perm] = np.arange(N)
+        X, el = X[perm], inv[el]
+    if repeat:                                    # a wedge: edge 4-7 of the last element collapsed onto node 4
+        el = el.copy()
+        el[-1, 7] = el[-1, 4]
+    mask = np.full(N, 7, np.uint8)
+    mask[0], mask[N // 2] = 0, 5
+    P = DevicePlan(X, mask, [("C3D8", el)])
+    h = 1.0 / max(dims)
+    gc = torch.from_numpy(rng.normal(0, 0.02 * h, P.ndof)).cuda()
+    return P, gc
+
+
+def close(a, b):
+    s = float(b.abs().max())
+    return float((a - b).abs().max()) <= TOL * s
+
+
+@pytest.mark.parametrize("dims", MESHES)
+@pytest.mark.parametrize("acc", [0, 1])
+@pytest.mark.parametrize("repeat", [False, True])
+def test_residual(dims, acc, repeat):
+    from fea_b200 import _lib as L
+    P, gc = hex_plan(dims, repeat=repeat)
+    g = P.groups[0]
+    n = int(L.fea_force_work_len(C.byref(g.desc)))
+    assert n == g.ne * 32
+    pad = torch.full((n + 64,), 7.25, dtype=torch.float64, device="cuda")
+    base = torch.linspace(-1, 1, P.ndof, dtype=torch.float64, device="cuda")
+    out = []
+    for w, wn in ((None, 0), (pad, n - 1), (pad, n)):
+        R, eR = base.clone(), torch.zeros(24 * g.ne, dtype=torch.float64, device="cuda")
+        L.check(L.fea_assemble_volume(C.byref(P.nodes), C.byref(g.desc), 1.0, 40.0, ptr(gc), None, ptr(R), ptr(eR), acc,
+                                      ptr(w), wn, stream()), "force")
+        out.append((R - base if acc else R, eR))
+        if wn < n:                                # too short a buffer is left alone
+            assert bool((pad == 7.25).all())
+    assert bool((pad[n:] == 7.25).all())
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert close(out[2][1], out[0][1])            # element residuals
+    if acc:                                       # (the sums are rounded to the base's size)
+        assert float((out[2][0] - out[0][0]).abs().max()) <= TOL * max(1.0, float(out[0][0].abs().max()))
+    else:
+        assert close(out[2][0], out[0][0])
+
+
+def test_residual_on_streams_and_under_capture():
+    """The plan's own buffer serves its own stream; other streams and a
+    capture take their own, with the same bits."""
+    P, gc = hex_plan((6, 5, 4))
+    ref = P.zeros(P.ndof)
+    P.assemble_volume(0, 1.0, 40.0, gc, R=ref)
+    torch.cuda.synchronize()
+    side, outs = torch.cuda.Stream(), []
+    side.wait_stream(torch.cuda.current_stream())
+    for k in range(8):                            # interleaved launches on two streams
+        a, b = P.zeros(P.ndof), P.zeros(P.ndof)
+        side.wait_stream(torch.cuda.current_stream())
+        P.assemble_volume(0, 1.0, 40.0, gc, R=a)
+        with torch.cuda.stream(side):
+            P.assemble_volume(0, 1.0, 40.0, gc, R=b)
+        outs += [a, b]
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, ref) for o in outs)
+    R = P.zeros(P.ndof)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        P.assemble_volume(0, 1.0, 40.0, gc, R=R)
+    R.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(R, ref)
+
+
+def test_residual_matches_the_oracle():
+    X, el = O.hex_block(3, jitter=0.1, seed=2)
+    from fea_b200 import DevicePlan
+    N = X.shape[0]
+    P = DevicePlan(X, np.full(N, 7, np.uint8), [("C3D8", el.numpy())])
+    gc = 1e-2 * torch.randn(3 * N, generator=torch.Generator().manual_seed(1), dtype=torch.float64)
+    R = P.zeros(P.ndof)
+    P.assemble_volume(0, 1.0, 40.0, gc.cuda(), R=R)
+    m = O.Model(X, [O.Group("C3D8", el, 1.0, 40.0)], [], [])
+    assert close(R.cpu(), m.assemble(gc, want_K=False)[0])
