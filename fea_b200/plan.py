@@ -155,7 +155,8 @@ class GatherGroup:
                             hp.scalar(L.FEA_S_G_HXSTRIDE, index) if uptr.size else 0)
         self.nchunk = int(self.desc.nchunk)
         # doubles of the element-once kernels' slots (C3D8 elements)
-        self.slot_len = int(L.fea_force_work_len(C.byref(self.desc))) if base == L.G_BASE else 0
+        self.slot_len = (max(int(L.fea_force_work_len(C.byref(self.desc))), int(L.fea_adjoint_work_len(C.byref(self.desc))))
+                         if base == L.G_BASE and kind == L.FEA_C3D8 and self.ne else 0)
 
 
 class DevicePlan:
@@ -318,10 +319,14 @@ class DevicePlan:
     def adjoint_vjp_volume(self, gi, mu, kappa, gc, lam_full, dX, dmu):
         """dX += d(lam . R_e)/dX (all nodes); dmu[0] = d(lam . R_e)/dmu."""
         g = self.groups[gi]
-        s = self.scratch(L.fea_reduce_scratch_len(g.ne))
-        L.check(L.fea_adjoint_vjp_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
-                                         vptr(lam_full), vptr(dX), vptr(dmu), vptr(s), s.numel(), stream()),
-                "fea_adjoint_vjp_volume")
+        s, n, lock = self.slots(g.slot_len) if g.slot_len else (None, 0, _NO_LOCK)
+        if s is None:
+            s = self.scratch(L.fea_reduce_scratch_len(g.ne))
+            n = s.numel()
+        with lock:
+            L.check(L.fea_adjoint_vjp_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
+                                             vptr(lam_full), vptr(dX), vptr(dmu), vptr(s), int(n), stream()),
+                    "fea_adjoint_vjp_volume")
 
     def adjoint_hvp_pressure(self, fi, p, Xinst, gc, v_full, out):
         """out += p d2V/dx2 v (all nodes) for face group fi."""

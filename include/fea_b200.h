@@ -521,10 +521,13 @@ int fea_explicit_run(const fea_nodes_t* nodes, const fea_group_t* group, double 
  *   fea_adjoint_vjp_volume: for the adjoint field lam [N,3] (all nodes,
  *     zero on Dirichlet DOFs) adds d(lam . R_e)/dX [N,3] to dX_dev (every
  *     node, constrained ones included) and writes d(lam . R_e)/dmu to
- *     dmu_dev[0].  scratch: fea_reduce_scratch_len(ne) doubles.
+ *     dmu_dev[0].  scratch: fea_reduce_scratch_len(ne) doubles at least;
+ *     with fea_adjoint_work_len(group) doubles, 16-byte aligned, a C3D8
+ *     group's elements are evaluated once each (else once per node).
  *   fea_adjoint_hvp_pressure: adds p d2V/dx2 v (all nodes) to out_dev, the
  *     X-derivative of v . (p dV/dx) of a pressure face group.
  * ------------------------------------------------------------------------- */
+int64_t fea_adjoint_work_len(const fea_group_t* group);
 int fea_adjoint_vjp_volume(const fea_nodes_t* nodes, const fea_group_t* group, double mu, double kappa,
                            const double* gc_dev, const double* lam_dev, double* dX_dev, double* dmu_dev,
                            double* scratch_dev, int64_t scratch_len, cudaStream_t stream);

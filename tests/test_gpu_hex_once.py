@@ -125,3 +125,26 @@ def test_residual_matches_the_oracle():
     P.assemble_volume(0, 1.0, 40.0, gc.cuda(), R=R)
     m = O.Model(X, [O.Group("C3D8", el, 1.0, 40.0)], [], [])
     assert close(R.cpu(), m.assemble(gc, want_K=False)[0])
+
+
+@pytest.mark.parametrize("dims", MESHES)
+@pytest.mark.parametrize("repeat", [False, True])
+def test_vjp(dims, repeat):
+    from fea_b200 import _lib as L
+    P, gc = hex_plan(dims, repeat=repeat)
+    g = P.groups[0]
+    n = int(L.fea_adjoint_work_len(C.byref(g.desc)))
+    lam = torch.randn(P.n_nodes, 3, dtype=torch.float64, generator=torch.Generator().manual_seed(4)).cuda()
+    pad = torch.full((n + 64,), 7.25, dtype=torch.float64, device="cuda")
+    short = int(L.fea_reduce_scratch_len(g.ne))
+    out = []
+    for wn in (short, n):
+        dX = torch.zeros(P.n_nodes, 3, dtype=torch.float64, device="cuda")
+        dmu = torch.zeros(1, dtype=torch.float64, device="cuda")
+        L.check(L.fea_adjoint_vjp_volume(C.byref(P.nodes), C.byref(g.desc), 1.0, 40.0, ptr(gc), ptr(lam), ptr(dX),
+                                         ptr(dmu), ptr(pad), wn, stream()), "vjp")
+        assert bool((pad[wn:] == 7.25).all())
+        out.append((dX, dmu))
+    assert close(out[1][0], out[0][0])
+    # a sum of 8 ne signed terms: against the sum of their sizes' bound
+    assert abs(float(out[1][1] - out[0][1])) <= TOL * max(float(out[0][1].abs()), g.ne * 1e-2)
