@@ -132,7 +132,7 @@ __device__ __forceinline__ void adj_M(const double F[9], const double iF[9], dou
 }
 
 // ---- C3D8: each element once (hexlane.cuh), dPhi/dmu in the same pass -------
-// Bound by FP64 issue and shared-memory reads.  40^3 block: 38.4 us + 7.2 us for
+// Bound by FP64 issue and shared-memory reads.  40^3 block: 38.4 us + 5.4 us for
 // the sum and 3.2 us for dPhi/dmu, against 286 us (k_vjp_vol<8>) and 28.7 us (k_vjp_mu<8>).
 __global__ void __launch_bounds__(HL_TPB, 4) k_hex_vjp(AdjParams P, double* __restrict__ slot,
                                                       double* __restrict__ partial) {
@@ -186,13 +186,11 @@ __global__ void __launch_bounds__(HL_TPB, 4) k_hex_vjp(AdjParams P, double* __re
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-__global__ void __launch_bounds__(128) k_hex_vjp_sum(AdjParams P, const double* __restrict__ slot) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= P.n_nodes) return;
-  double r[3];
-  hex_sum_slots(slot, P.allinc, P.allptr[n], P.allptr[n + 1], r);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) P.out[3 * (int64_t)n + i] += r[i];
+__global__ void __launch_bounds__(HL_SUM_TPB) k_hex_vjp_sum(AdjParams P, const double* __restrict__ slot) {
+  const int64_t t = (int64_t)blockIdx.x * HL_SUM_TPB + threadIdx.x;
+  const int n = (int)(t >> 2), j = (int)(t & 3);
+  if (n >= P.n_nodes || j == 3) return;
+  P.out[3 * (int64_t)n + j] += hex_sum_slots(slot, P.allinc, P.allptr[n], P.allptr[n + 1], j);
 }
 
 // dPhi/dX for every node: one thread per node over all its incidences (C3D4,
@@ -385,7 +383,7 @@ extern "C" int fea_adjoint_vjp_volume(const fea_nodes_t* N, const fea_group_t* G
     const int64_t nb = (G->ne + HL_EPB - 1) / HL_EPB;
     double* partial = scratch + G->ne * 8 * HL_SLOT;
     k_hex_vjp<<<(unsigned)nb, HL_TPB, 0, st>>>(P, scratch, partial);
-    k_hex_vjp_sum<<<grid_for(N->n_nodes, 128), 128, 0, st>>>(P, scratch);
+    k_hex_vjp_sum<<<hex_sum_grid(N->n_nodes), HL_SUM_TPB, 0, st>>>(P, scratch);
     k_sum_partials_adj<<<1, 256, 0, st>>>(partial, nb, dmu);
     count_launch(3);
     return (int)cudaGetLastError();

@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(HX_GW * 32, 8) k_hex_gat(VolParams P, const do
 // ---- C3D8 R only: each element once, then a sum per node --------------------
 // (hexlane.cuh has the scheme.)  Bound by FP64 issue and shared-memory reads:
 // about 420 FP64 operations a Gauss point (20 us of FP64 issue for the 48^3
-// block).  48^3 block: 37.3 us + 10 us for the sum, against 366 us with a
+// block).  48^3 block: 37.3 us + 7.3 us for the sum, against 366 us with a
 // thread per node (k_vol_r<8>); five CTAs per SM (8 bytes of spills) 37.3
 // against 38.3 us with four.
 template <bool ER>
@@ -814,21 +814,15 @@ __global__ void __launch_bounds__(HL_TPB, 5) k_hex_force(VolParams P, double* __
 }
 
 template <bool ACC>
-__global__ void __launch_bounds__(128) k_hex_force_sum(VolParams P, const double* __restrict__ slot) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= P.n_nodes) return;
+__global__ void __launch_bounds__(HL_SUM_TPB) k_hex_force_sum(VolParams P, const double* __restrict__ slot) {
+  const int64_t t = (int64_t)blockIdx.x * HL_SUM_TPB + threadIdx.x;
+  const int n = (int)(t >> 2), j = (int)(t & 3);
+  if (n >= P.n_nodes || j == 3) return;
   const unsigned mn = P.mask[n];
-  if (!mn) return;
-  double r[3];
-  hex_sum_slots(slot, P.inc, P.nodeinc[n], P.nodeinc[n + 1], r);
-  double* Rout = P.R + P.rdof[n];
-  int rj = 0;
-#pragma unroll
-  for (int j = 0; j < 3; ++j)
-    if (mn >> j & 1u) {
-      Rout[rj] = ACC ? Rout[rj] + r[j] : r[j];
-      ++rj;
-    }
+  if (!(mn >> j & 1u)) return;
+  const double r = hex_sum_slots(slot, P.inc, P.nodeinc[n], P.nodeinc[n + 1], j);
+  double* out = P.R + P.rdof[n] + rank3(mn, j);
+  *out = ACC ? *out + r : r;
 }
 
 // R-only kernel: one thread per node, sequential over its incidences (C3D4,
@@ -1629,8 +1623,9 @@ extern "C" int fea_assemble_volume(const fea_nodes_t* N, const fea_group_t* G, d
     const unsigned eg = (unsigned)((G->ne + HL_EPB - 1) / HL_EPB);
     if (elemR) k_hex_force<true><<<eg, HL_TPB, 0, st>>>(P, work);
     else k_hex_force<false><<<eg, HL_TPB, 0, st>>>(P, work);
-    if (accumulate) k_hex_force_sum<true><<<grid, 128, 0, st>>>(P, work);
-    else k_hex_force_sum<false><<<grid, 128, 0, st>>>(P, work);
+    const unsigned sg = hex_sum_grid(N->n_nodes);
+    if (accumulate) k_hex_force_sum<true><<<sg, HL_SUM_TPB, 0, st>>>(P, work);
+    else k_hex_force_sum<false><<<sg, HL_SUM_TPB, 0, st>>>(P, work);
     count_launch(2);
     return (int)cudaGetLastError();
   }

@@ -19,6 +19,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "hexlane.cuh"
 
 namespace fea {
 
@@ -102,6 +103,101 @@ __device__ __forceinline__ void elem_force(const ExParams& P, const int32_t* cn,
   }
 }
 
+// Central-difference update of the free component d of node n (mask mn) from
+// its force r (flags as at k_explicit); returns its displacement at u_{k+1}
+// when it advances.
+__device__ __forceinline__ double advance_dof(const ExParams& P, int32_t base, unsigned mn, int d, double r, int flags) {
+  const int32_t i = base + rank3(mn, d);
+  const double acc = (flags & 1) ? -P.minv[i] * r : P.a[i];
+  if (flags & 1) P.a[i] = acc;
+  if (flags & 4) {
+    const double vh = (flags & 2) ? P.vh[i] - 0.5 * P.dt * acc : P.vh[i];
+    const double vhn = vh + P.dt * acc;
+    P.v[i] = 0.5 * (vhn + vh);
+    P.vh[i] = vhn;
+    const double un = P.u[i] + P.dt * vhn;
+    P.unext[i] = un;
+    return un;
+  }
+  if (flags & 2) P.vh[i] = P.vh[i] - 0.5 * P.dt * acc;
+  return 0.0;
+}
+
+// ---- C3D8: each element once (hexlane.cuh), then the nodes -------------------
+// k_hex_exforce<T> evaluates the elements in T and writes the nodal forces
+// (formed in FP64) to the elements' slots; k_hex_exnode sums a node's slots
+// and advances it.  Bound by FP64 issue and shared-memory reads (FP32: the
+// latter).  40^3 block, per step: 20.9 + 6.3 us, against 148 us for k_explicit<8>
+// (FP64).
+template <class T>
+__global__ void __launch_bounds__(HL_TPB, 5) k_hex_exforce(ExParams P, int64_t ne, double* __restrict__ slot) {
+  __shared__ __align__(16) double sv[HL_EPB * HL_EL];
+  const int le = threadIdx.x >> 3, lane = threadIdx.x & 7;
+  const int64_t e = (int64_t)blockIdx.x * HL_EPB + le;
+  const bool act = e < ne;
+  double* V = sv + le * HL_EL;
+  if (act) {
+    const double2* xb = reinterpret_cast<const double2*>(P.xu + 6 * (int64_t)P.conn[e * 8 + lane]);
+    double2* o = reinterpret_cast<double2*>(V + 6 * lane);
+    o[0] = xb[0];
+    o[1] = xb[1];
+    o[2] = xb[2];
+  }
+  __syncwarp();
+  T JJ[2][9];
+  {
+    const HexLane<T> H(lane);
+    if (act) hex_gradients<T, 2>(H, V, JJ);
+  }
+  __syncwarp();                                  // the node data are read: the area takes the matrices
+  if (act) {
+    T iJ[9], F[9], iF[9], M[9], J, Jm;
+    const T w = inv3(JJ[0], iJ);                 // Gauss weight 1
+    const T* Ju = JJ[1];
+#pragma unroll
+    for (int I = 0; I < 3; ++I)
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        F[3 * I + i] = (I == i ? T(1) : T(0)) + Ju[3 * I] * iJ[i] + Ju[3 * I + 1] * iJ[3 + i] + Ju[3 * I + 2] * iJ[6 + i];
+    if constexpr (sizeof(T) == 8) {
+      double jmd;
+      J = inv3_jm(F, iF, &jmd);
+      Jm = jmd;
+    } else {
+      J = inv3(F, iF);
+      Jm = (T)jm23((double)J);
+    }
+    T sF2 = T(0);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) sF2 += F[i] * F[i];
+    const T muJm = (T)P.mu * Jm, c2 = (T)P.kappa * J * (J - T(1)) - (T)P.mu * (Jm * sF2) / T(3);
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) M[3 * j + i] = muJm * F[3 * j + i] + c2 * iF[3 * i + j];
+    hex_put(V, lane, w, M, iJ);
+  }
+  __syncwarp();
+  if (!act) return;
+  const HexLane<double> H(lane);
+  double r[3];
+  hex_take(H, V, lane, r);
+  hex_store_slot(slot, e, lane, r);
+}
+
+__global__ void __launch_bounds__(HL_SUM_TPB) k_hex_exnode(ExParams P, const double* __restrict__ slot, int flags) {
+  const int64_t t = (int64_t)blockIdx.x * HL_SUM_TPB + threadIdx.x;
+  const int n = (int)(t >> 2), d = (int)(t & 3);
+  if (n >= P.n_nodes || d == 3) return;
+  const unsigned mn = P.mask[n];
+  double un = 0.0;                               // (fixed components stay 0)
+  if (mn >> d & 1u) {
+    const double r = (flags & 1) ? hex_sum_slots(slot, P.inc, P.nodeinc[n], P.nodeinc[n + 1], d) : 0.0;
+    un = advance_dof(P, P.rdof[n], mn, d, r, flags);
+  }
+  if ((flags & 4) && mn) P.xunext[6 * (int64_t)n + 3 + d] = un;   // the node's copy at u_{k+1}
+}
+
 // flags: bit0 compute the force (else use a), bit1 init (vh = v0 - dt/2 a),
 //        bit2 advance (vh, v, u_next)
 template <int NN, class T>
@@ -146,25 +242,10 @@ __global__ void __launch_bounds__(128, NN == 4 ? 5 : 1) k_explicit(ExParams P, i
     }
   }
   const int32_t base = P.rdof[n];
-  int rj = 0;
   double un[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    if (!(mn >> d & 1u)) continue;
-    const int32_t i = base + rj++;
-    double acc = (flags & 1) ? -P.minv[i] * r[d] : P.a[i];
-    if (flags & 1) P.a[i] = acc;
-    if (flags & 4) {
-      double vh = (flags & 2) ? P.vh[i] - 0.5 * P.dt * acc : P.vh[i];
-      double vhn = vh + P.dt * acc;
-      P.v[i] = 0.5 * (vhn + vh);
-      P.vh[i] = vhn;
-      un[d] = P.u[i] + P.dt * vhn;
-      P.unext[i] = un[d];
-    } else if (flags & 2) {
-      P.vh[i] = P.vh[i] - 0.5 * P.dt * acc;
-    }
-  }
+  for (int d = 0; d < 3; ++d)
+    if (mn >> d & 1u) un[d] = advance_dof(P, base, mn, d, r[d], flags);
   if (flags & 4) {                               // the node's copy at u_{k+1} (fixed components 0)
     double* o = P.xunext + 6 * (int64_t)n;
     o[3] = un[0];
@@ -241,6 +322,11 @@ extern "C" int64_t fea_explicit_work_len(const fea_nodes_t* N) {
   return ((N->ndof + 1) & ~(int64_t)1) + 12 * N->n_nodes;
 }
 
+extern "C" int64_t fea_explicit_group_work_len(const fea_nodes_t* N, const fea_group_t* G) {
+  const int64_t base = fea_explicit_work_len(N);
+  return G && G->kind == FEA_C3D8 && G->ne > 0 ? base + G->ne * 8 * HL_SLOT : base;
+}
+
 // state on entry: u = u_k, vh = vh_{k-1/2}, a = a_k   (init == 0), or
 //                 u = u_0, v = v_0 (a, vh are outputs)  (init != 0)
 extern "C" int fea_explicit_run(const fea_nodes_t* N, const fea_group_t* G, double mu, double kappa,
@@ -274,12 +360,22 @@ extern "C" int fea_explicit_run(const fea_nodes_t* N, const fea_group_t* G, doub
   count_launch();
   const int grid = grid_for(N->n_nodes, 128);
   const bool hex = G->kind == FEA_C3D8;
+  const bool once = hex && G->ne > 0 && work_len >= fea_explicit_group_work_len(N, G);
+  double* slot = work + fea_explicit_work_len(N);
   auto launch = [&](const double* ucur, double* unext, int flags) {
     P.u = ucur;
     P.unext = unext;
     P.xu = xub[ucur == u ? 0 : 1];
     P.xunext = xub[ucur == u ? 1 : 0];
-    if (hex) {
+    if (once) {
+      if (flags & 1) {
+        const unsigned eg = (unsigned)((G->ne + HL_EPB - 1) / HL_EPB);
+        if (fp32) k_hex_exforce<float><<<eg, HL_TPB, 0, st>>>(P, G->ne, slot);
+        else k_hex_exforce<double><<<eg, HL_TPB, 0, st>>>(P, G->ne, slot);
+        count_launch();
+      }
+      k_hex_exnode<<<hex_sum_grid(N->n_nodes), HL_SUM_TPB, 0, st>>>(P, slot, flags);
+    } else if (hex) {
       if (fp32) k_explicit<8, float><<<grid, 128, 0, st>>>(P, flags);
       else k_explicit<8, double><<<grid, 128, 0, st>>>(P, flags);
     } else {

@@ -129,33 +129,27 @@ __device__ __forceinline__ void hex_store_slot(double* __restrict__ slot, int64_
   o[1] = make_double2(r[2], 0.0);
 }
 
-// Sum of the slots of the incidences inc[q0 .. q1) (element * 16 + local
-// node, element order ascending): the loads of the 8 incidences of an
-// interior node are issued together.
-__device__ __forceinline__ void hex_sum_slots(const double* __restrict__ slot, const int32_t* __restrict__ inc, int q0,
-                                              int q1, double r[3]) {
+// Component j of the sum of the slots of the incidences inc[q0 .. q1)
+// (element * 16 + local node, element order ascending).  Four threads per
+// node, one per component and one idle: with a thread per node the sum waited
+// on one load after the other at 15 warps per SM (48^3 block: 10.7 -> 7.3 us).
+constexpr int HL_SUM_TPB = 256;
+__device__ __forceinline__ double hex_sum_slots(const double* __restrict__ slot, const int32_t* __restrict__ inc,
+                                                int q0, int q1, int j) {
   constexpr int U = 8;
-  r[0] = r[1] = r[2] = 0.0;
+  double r = 0.0;
   for (int q = q0; q < q1; q += U) {
     int ea[U];
-    double2 a[U];
-    double c[U];
+    double v[U];
 #pragma unroll
     for (int k = 0; k < U; ++k) ea[k] = inc[min(q + k, q1 - 1)];   // (past the end: the last one, not added)
 #pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const double* s = slot + ((int64_t)(ea[k] >> 4) * 8 + (ea[k] & 15)) * HL_SLOT;
-      a[k] = *reinterpret_cast<const double2*>(s);
-      c[k] = s[2];
-    }
+    for (int k = 0; k < U; ++k) v[k] = slot[((int64_t)(ea[k] >> 4) * 8 + (ea[k] & 15)) * HL_SLOT + j];
 #pragma unroll
-    for (int k = 0; k < U; ++k)
-      if (q + k < q1) {
-        r[0] += a[k].x;
-        r[1] += a[k].y;
-        r[2] += c[k];
-      }
+    for (int k = 0; k < U; ++k) r += q + k < q1 ? v[k] : 0.0;
   }
+  return r;
 }
+inline unsigned hex_sum_grid(int64_t n_nodes) { return (unsigned)((n_nodes * 4 + HL_SUM_TPB - 1) / HL_SUM_TPB); }
 
 }  // namespace fea

@@ -148,3 +148,33 @@ def test_vjp(dims, repeat):
     assert close(out[1][0], out[0][0])
     # a sum of 8 ne signed terms: against the sum of their sizes' bound
     assert abs(float(out[1][1] - out[0][1])) <= TOL * max(float(out[0][1].abs()), g.ne * 1e-2)
+
+
+@pytest.mark.parametrize("dims", MESHES)
+@pytest.mark.parametrize("fp32", [0, 1])
+def test_explicit_steps(dims, fp32):
+    """A start and five steps: the C ABI with the short work buffer (the
+    per-node path) and with the slots."""
+    from fea_b200 import _lib as L
+    P, gc = hex_plan(dims)
+    g = P.groups[0]
+    minv = P.lumped_mass_inv([1.0])
+    short = int(L.fea_explicit_work_len(C.byref(P.nodes)))
+    n = int(L.fea_explicit_group_work_len(C.byref(P.nodes), C.byref(g.desc)))
+    assert n == short + 32 * g.ne
+    v0 = 0.01 * torch.randn(P.ndof, dtype=torch.float64, generator=torch.Generator().manual_seed(5)).cuda()
+    dt = 0.02 / max(dims)
+    out = []
+    for wn in (short, n):
+        pad = torch.full((wn + 64,), 7.25, dtype=torch.float64, device="cuda")
+        u, v, vh, a = gc.clone(), v0.clone(), torch.empty_like(gc), torch.empty_like(gc)
+        for init, steps in ((1, 2), (0, 3)):
+            L.check(L.fea_explicit_run(C.byref(P.nodes), C.byref(g.desc), 1.0, 40.0, ptr(minv), dt, steps, fp32, init,
+                                       ptr(u), ptr(vh), ptr(a), ptr(v), ptr(pad), wn, stream()), "explicit")
+        assert bool((pad[wn:] == 7.25).all())
+        out.append((u, v, a))
+    # FP32 element math: the accelerations' error is kappa * 6e-8 of the stresses' scale per Gauss point
+    # (3e-5 of the largest acceleration, either path)
+    tol = 1e-4 if fp32 else TOL * 10
+    for x, y in zip(*out):
+        assert float((x - y).abs().max()) <= tol * float(x.abs().max())
