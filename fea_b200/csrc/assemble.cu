@@ -247,10 +247,221 @@ __device__ __forceinline__ void write_back(const int32_t* __restrict__ chunkptr,
   }
 }
 
+// ---- C3D4 R + K ---------------------------------------------------------------
+// One CTA per tile of consecutive node rows.  A thread evaluates the element
+// of one incidence (row node a) and leaves its strip K_e[a, :] (4 blocks of
+// 9) and R_a in shared memory.  Then a thread takes one neighbour block of a node: it
+// sums the contributions that the plan lists for it (CREC, CLIST, in
+// incidence order) and writes the block's 3 x 3 values; the node's own block
+// and residual, to which every incidence contributes (24 instead of 4 to 6),
+// take a thread per value.  Every K value is written once.
+// Bound by latency at the 16 warps per SM that 122 registers leave (each
+// element is evaluated by 4 threads: 21 us of FP64 issue for the 190k-element
+// beam), by the scattered node loads and by shared-memory bank conflicts of
+// the contributions.  190k-element beam: 79.8 us, against 393 us with the
+// strips summed in rounds, one incidence of each node at a time (k_vol_rk);
+// 256-thread tiles 84.5; node data staged once per tile 75.8, not worth its
+// share of the plan (13 ms a 30k-element beam); nine lanes per block 105; a
+// thread per value 111 to 121.
+struct TetLists {
+  const uint16_t* __restrict__ clist;
+  const uint2* __restrict__ crec;
+  const int64_t* __restrict__ crecptr;
+  const int32_t* __restrict__ tileptr;
+};
+struct alignas(16) TetNode {               // a node of the chunk
+  int64_t vbase;
+  int32_t e0, r0, ni, L, dbase, off;   // e0: its first block of the chunk's; off: its own columns in its rows
+  uint32_t mask, list;                 // list: its own part of CLIST
+};
+constexpr int TET_TPB = FEA_TET_TILE;
+constexpr int TET_ST = FEA_TET_STRIDE;       // odd: a warp's strided stores fall on all banks
+constexpr size_t TET_SMEM = sizeof(double) * TET_TPB * TET_ST + sizeof(TetNode) * (TET_TPB + 1) +
+                            sizeof(uint16_t) * TET_TPB * 4;   // strips, node records, codes
+
+// strip of local node a: 4 blocks of 9 to C, then R_a
+__device__ __forceinline__ void tet_strip(const VolParams& P, const int32_t cn[4], int a, double* C) {
+  double x[4][3], u[4][3];
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const unsigned m = P.mask[cn[b]];
+    const int32_t rd = P.rdof[cn[b]];
+    const double* xb = P.X + 3 * (int64_t)cn[b];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      x[b][i] = __ldg(xb + i);
+      u[b][i] = node_u(P.gc, rd, m, i);
+    }
+  }
+  double J0[9], iJ[9], F[9], iF[9], Ju[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      J0[3 * i + m] = x[m + 1][i] - x[0][i];
+      Ju[3 * i + m] = u[m + 1][i] - u[0][i];
+    }
+  const double w = inv3(J0, iJ) * Elem<4>::wq(0);
+#pragma unroll
+  for (int I = 0; I < 3; ++I)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      F[3 * I + i] = fma(Ju[3 * I], iJ[i], fma(Ju[3 * I + 1], iJ[3 + i], fma(Ju[3 * I + 2], iJ[6 + i], I == i ? 1.0 : 0.0)));
+  double Jm;
+  const double J = inv3_jm(F, iF, &Jm);
+  const double mu = P.mu, kappa = P.kappa;
+  double sF2 = 0.0;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) sF2 += F[i] * F[i];
+  const double I1 = Jm * sF2, muJm = mu * Jm;
+  const double wa = w * (-2.0 / 3.0 * muJm), wb = w * (kappa * J * (2.0 * J - 1.0) + 2.0 / 9.0 * mu * I1),
+               wg = w * (mu * I1 / 3.0 - kappa * J * (J - 1.0)), wc = w * muJm,
+               wc2 = w * (kappa * J * (J - 1.0) - mu * I1 / 3.0);
+  // q_b = F^-T g_b, f_b = F g_b; node 0's gradient is minus the sum of the others
+  double q[4][3], f[4][3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      q[m + 1][k] = iJ[3 * m] * iF[k] + iJ[3 * m + 1] * iF[3 + k] + iJ[3 * m + 2] * iF[6 + k];
+      f[m + 1][k] = iJ[3 * m] * F[3 * k] + iJ[3 * m + 1] * F[3 * k + 1] + iJ[3 * m + 2] * F[3 * k + 2];
+    }
+    q[0][k] = -(q[1][k] + q[2][k] + q[3][k]);
+    f[0][k] = -(f[1][k] + f[2][k] + f[3][k]);
+  }
+  double A[3], B[3], G[3], S[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double qa = a < 2 ? (a ? q[1][k] : q[0][k]) : (a == 2 ? q[2][k] : q[3][k]);
+    const double fa = a < 2 ? (a ? f[1][k] : f[0][k]) : (a == 2 ? f[2][k] : f[3][k]);
+    A[k] = wa * fa + wb * qa;
+    B[k] = wa * qa;
+    G[k] = wg * qa;
+    S[k] = wc * fa;                              // w mu J^-2/3 f_a: delta term S . q_b
+    C[36 + k] = S[k] + wc2 * qa;
+  }
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const double dg = S[0] * q[b][0] + S[1] * q[b][1] + S[2] * q[b][2];
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        C[9 * b + 3 * j + k] = fma(A[j], q[b][k], fma(B[j], f[b][k], fma(q[b][j], G[k], j == k ? dg : 0.0)));
+  }
+}
+
+template <bool WR, bool ACC, bool ER>
+__global__ void __launch_bounds__(TET_TPB, 4) k_tet_rk(VolParams P, TetLists T) {
+  extern __shared__ __align__(16) double sm[];
+  TetNode* nodes = reinterpret_cast<TetNode*>(sm + TET_TPB * TET_ST);
+  uint16_t* codes = reinterpret_cast<uint16_t*>(nodes + TET_TPB + 1);
+  const int tid = threadIdx.x;
+  const int ch = blockIdx.x;
+  const int l0 = T.tileptr[ch], nl = T.tileptr[ch + 1] - l0;   // nodes (each has an incidence)
+  const int na = P.chunklist[l0], nz = P.chunklist[l0 + nl - 1];
+  const int i0 = P.nodeinc[na], ni = P.nodeinc[nz + 1] - i0;     // incidences
+  const int64_t c0 = T.crecptr[na];              // the tile's records are contiguous
+  for (int l = tid; l <= nl; l += TET_TPB) {
+    TetNode d{};
+    const int n = P.chunklist[l0 + min(l, nl - 1)];
+    if (l < nl) {
+      const int64_t c = T.crecptr[n];
+      const uint2 self = T.crec[c];
+      d.vbase = P.vbase[n];
+      d.e0 = (int)(c - c0);
+      d.r0 = P.nodeinc[n] - i0;
+      d.ni = P.nodeinc[n + 1] - P.nodeinc[n];
+      d.L = P.rowlen[n];
+      d.dbase = P.dbase[n];
+      d.off = (int)(self.x & 0xffffu);
+      d.mask = self.x >> 16;
+      d.list = self.y;
+    } else {
+      d.e0 = (int)(T.crecptr[n + 1] - c0);
+    }
+    nodes[l] = d;
+  }
+  for (int i = tid; i < ni; i += TET_TPB)        // the chunk's codes are contiguous
+    reinterpret_cast<uint2*>(codes)[i] = reinterpret_cast<const uint2*>(T.clist)[i0 + i];
+  if (tid < ni) {
+    const int ea = P.inc[i0 + tid];
+    const int64_t e = ea >> 4;
+    const int a = ea & 15;
+    const int4 c = *reinterpret_cast<const int4*>(P.conn + 4 * e);
+    const int32_t cn[4] = {c.x, c.y, c.z, c.w};
+    double* C = sm + tid * TET_ST;
+    tet_strip(P, cn, a, C);
+    if (ER) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) P.elemR[(int64_t)(3 * a + j) * P.ne + e] = C[36 + j];
+    }
+  }
+  __syncthreads();
+  // the blocks of the tile, then 12 values per node (its own block, residual)
+  const int ne = nodes[nl].e0;
+  for (int i = tid, l = 0; i < ne + 12 * nl; i += TET_TPB) {
+    if (i < ne) {
+      while (i >= nodes[l + 1].e0) ++l;
+      const TetNode& d = nodes[l];
+      if (i == d.e0) continue;
+      const uint2 rec = T.crec[c0 + i];
+      const double* C = sm + d.r0 * TET_ST;
+      const uint16_t* code = codes + 4 * d.r0 + (rec.y & 0x7ffu);
+      const int cnt = (int)(rec.y >> 11);
+      double s[9];
+#pragma unroll
+      for (int t = 0; t < 9; ++t) s[t] = 0.0;
+#pragma unroll 2
+      for (int k = 0; k < cnt; ++k) {
+        const double* v = C + code[k];
+#pragma unroll
+        for (int t = 0; t < 9; ++t) s[t] += v[t];
+      }
+      const unsigned mc = rec.x >> 16;
+      double* row = P.K + d.vbase + (rec.x & 0xffffu);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        if (!(d.mask >> j & 1u)) continue;
+        int rk = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (!(mc >> k & 1u)) continue;
+          row[rk] = ACC ? row[rk] + s[3 * j + k] : s[3 * j + k];
+          ++rk;
+        }
+        row += d.L;
+      }
+    } else {
+      const int q = i - ne;
+      const TetNode& d = nodes[q / 12];
+      const int c = q % 12, j = c < 9 ? c / 3 : c - 9, k = c - 3 * j;
+      if (!(d.mask >> j & 1u)) continue;
+      const double* C = sm + d.r0 * TET_ST;
+      double s = 0.0;
+      if (c < 9) {
+        if (!(d.mask >> k & 1u)) continue;
+        const uint16_t* code = codes + 4 * d.r0 + (d.list & 0x7ffu);
+        const int cnt = (int)(d.list >> 11);
+#pragma unroll 4
+        for (int r = 0; r < cnt; ++r) s += C[code[r] + c];
+        double* out = P.K + d.vbase + (int64_t)rank3(d.mask, j) * d.L + d.off + rank3(d.mask, k);
+        *out = ACC ? *out + s : s;
+      } else if (WR) {
+#pragma unroll 4
+        for (int r = 0; r < d.ni; ++r) s += C[r * TET_ST + 27 + c];
+        double* out = P.R + d.dbase + rank3(d.mask, j);
+        *out = ACC ? *out + s : s;
+      }
+    }
+  }
+}
+
 template <int NN>
 struct VolTPB { static constexpr int v = NN == 8 ? 128 : 256; };
 
-// R + K gather kernel: one CTA per chunk of consecutive node rows.
+// R + K in rank rounds, for a C3D4 descriptor without column lists: one CTA
+// per chunk of consecutive node rows.
 template <int NN, bool WR, bool ACC, bool ER>
 __global__ void __launch_bounds__(VolTPB<NN>::v) k_vol_rk(VolParams P) {
   extern __shared__ double sm[];
@@ -1606,6 +1817,23 @@ extern "C" int fea_assemble_volume(const fea_nodes_t* N, const fea_group_t* G, d
         gk<<<g2, HX_GW * 32, gbytes, st>>>(P, work, rslot, capb, capq);
         count_launch();
       }
+      return (int)cudaGetLastError();
+    }
+    // (16-byte loads of the connectivity, 8-byte ones of the lists)
+    if (G->clist_dev && G->crec_dev && G->crecptr_dev && G->tileptr_dev && ((uintptr_t)G->conn_dev & 15) == 0 &&
+        (((uintptr_t)G->clist_dev | (uintptr_t)G->crec_dev) & 7) == 0) {
+      if ((size_t)smem * sizeof(double) > (size_t)smem_limit()) return FEA_ESMEM;
+      if (G->ntile <= 0) return FEA_OK;
+      void (*k)(VolParams, TetLists) =
+          wr ? (acc ? (er ? k_tet_rk<true, true, true> : k_tet_rk<true, true, false>)
+                    : (er ? k_tet_rk<true, false, true> : k_tet_rk<true, false, false>))
+             : (acc ? (er ? k_tet_rk<false, true, true> : k_tet_rk<false, true, false>)
+                    : (er ? k_tet_rk<false, false, true> : k_tet_rk<false, false, false>));
+      if (cudaError_t ce = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TET_SMEM))
+        return (int)ce;
+      k<<<(unsigned)G->ntile, TET_TPB, TET_SMEM, st>>>(
+          P, TetLists{G->clist_dev, reinterpret_cast<const uint2*>(G->crec_dev), G->crecptr_dev, G->tileptr_dev});
+      count_launch();
       return (int)cudaGetLastError();
     }
 #define FEA_RK(NN_, WR_, ACC_, ER_)                                                                    \

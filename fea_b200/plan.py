@@ -59,6 +59,9 @@ class HostPlan:
             L.A_ROFF: np.int32, L.A_UPTR: np.int64, L.A_UBLK: np.int64, L.A_ALLPTR: np.int32,
             L.A_ALLINC: np.int32, L.A_INCPOS: np.int32, L.A_STAGEPOS: np.int32, L.A_REGION: np.int64}
 
+    _TDT = {L.FEA_A_G_CLIST: np.uint16, L.FEA_A_G_CREC: np.uint32, L.FEA_A_G_CRECPTR: np.int64,
+            L.FEA_A_G_TILEPTR: np.int32}
+
     def __init__(self, n_nodes, free_mask, groups, faces, vol_threads=0, smem_doubles=0):
         self._h = None
         mask = np.ascontiguousarray(free_mask, dtype=np.uint8)
@@ -94,7 +97,9 @@ class HostPlan:
         return int(v.value)
 
     def array(self, aid, group=0):
-        if aid >= L.F_BASE:
+        if aid in self._TDT:
+            dt = self._TDT[aid]
+        elif aid >= L.F_BASE:
             dt = self._GDT[aid - L.F_BASE]
         elif aid >= L.G_BASE:
             dt = self._GDT[aid - L.G_BASE]
@@ -135,6 +140,12 @@ class GatherGroup:
         self.region = dev(region) if uptr.size else None
         nblk = int(region[-1])
         maxblk = int(np.diff(region).max()) if region.size > 1 else 0
+        # neighbour lists of a C3D4 group (bit patterns: torch has no plain unsigned types)
+        self.lists = []
+        if base == L.G_BASE and hp.array(L.FEA_A_G_CRECPTR, index).size:
+            self.lists = [dev(hp.array(aid, index).view(vt)) for aid, vt in
+                          ((L.FEA_A_G_CLIST, np.int16), (L.FEA_A_G_CREC, np.int32), (L.FEA_A_G_CRECPTR, np.int64),
+                           (L.FEA_A_G_TILEPTR, np.int32))]
         self.allptr = dev(hp.array(base + L.A_ALLPTR, index))
         self.allinc = dev(hp.array(base + L.A_ALLINC, index))
         self.ne = int(self.conn.shape[0])
@@ -152,7 +163,9 @@ class GatherGroup:
                             self.incpos.data_ptr() if self.incpos is not None else None,
                             self.stagepos.data_ptr() if self.stagepos is not None else None,
                             self.region.data_ptr() if self.region is not None else None, nblk, maxblk,
-                            hp.scalar(L.FEA_S_G_HXSTRIDE, index) if uptr.size else 0)
+                            hp.scalar(L.FEA_S_G_HXSTRIDE, index) if uptr.size else 0,
+                            *([t.data_ptr() for t in self.lists] + [self.lists[-1].numel() - 1]
+                              if self.lists else []))
         self.nchunk = int(self.desc.nchunk)
         # doubles of the element-once kernels' slots (C3D8 elements)
         self.slot_len = (max(int(L.fea_force_work_len(C.byref(self.desc))), int(L.fea_adjoint_work_len(C.byref(self.desc))))

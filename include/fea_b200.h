@@ -51,6 +51,11 @@ extern "C" {
 #define FEA_ETOOBIG -8     /* size beyond a fixed limit: of an allocation-free entry point, or a
                               group of more than FEA_PLAN_MAX_ELEMS elements or faces */
 
+/* C3D4 assembly: incidences per tile (threads per CTA), and doubles per
+ * incidence in the kernel's shared memory (4 blocks of 9, residual 3) */
+#define FEA_TET_TILE 128
+#define FEA_TET_STRIDE 39
+
 /* element kinds (reference class names) */
 #define FEA_C3D4 4
 #define FEA_C3D8 8
@@ -126,6 +131,13 @@ enum {
   FEA_A_G_STAGEPOS = 48, /* int32 [ne, 36] staged block of each element block, -1: none  */
   FEA_A_G_REGION = 49,   /* int64 [N+1] first staged block of each node's region (even)   */
   FEA_S_G_HXSTRIDE = 70, /* int64 scalar: C3D8 fixed region stride in blocks, 0 = packed  */
+  FEA_A_G_CLIST = 71,    /* uint16 [ninc*4] C3D4: the node's contributions, neighbour by neighbour:
+                            offsets rank * FEA_TET_STRIDE + 9 b of incidence rank's block b */
+  FEA_A_G_CREC = 72,     /* uint32 pairs, one per neighbour of a node with rows (itself first): its
+                            columns' offset in the rows | free components << 16, and its part of
+                            the node's CLIST, start | count << 11                       */
+  FEA_A_G_CRECPTR = 73,  /* int64 [N+1] first neighbour record of each node    */
+  FEA_A_G_TILEPTR = 74,  /* int32 [ntile+1] C3D4 tiles: consecutive nodes of CHUNKLIST         */
   FEA_A_F_INC = 50,      /* the same arrays / scalars for face groups      */
   FEA_A_F_BOFF = 51,
   FEA_A_F_NODEINC = 52,
@@ -219,6 +231,11 @@ typedef struct {
                                  the fixed layout (regions at n * hx_stride =
                                  n * maxblk, records at 16 n, residual slots at
                                  n * maxval); 0: packed (REGION, UPTR, NODEINC) */
+  const uint16_t* clist_dev;  /* FEA_A_G_CLIST, _CREC, _CRECPTR, _TILEPTR     */
+  const uint32_t* crec_dev;   /* (C3D4 only); any NULL: the tangent is summed */
+  const int64_t* crecptr_dev; /* in rank rounds                               */
+  const int32_t* tileptr_dev;
+  int64_t ntile;
 } fea_group_t;
 
 /* Element residual and tangent of one Neo-Hookean group, gathered per node

@@ -1,0 +1,113 @@
+"""C3D4 tangent and residual by column lists (k_tet_rk) against the rank-round
+kernel, which the same entry point takes for a descriptor without lists:
+chunks with one and with many nodes, a node shared by 120 tetrahedra, partly
+fixed nodes, a doubled element, accumulate, no residual, and the
+element residual.  Each entry sums the same contributions in the same order;
+the strips differ by the rounding of 1/J (three roundings instead of a
+division) and of g_a . g_b: 1e-12 of the largest entry bounds it."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def ptr(t):
+    return None if t is None else C.c_void_p(t.data_ptr())
+
+
+def fan(n):
+    """n tetrahedra around the axis (0, 1): both axis nodes lie in all of them."""
+    t = 2 * np.pi * np.arange(n) / n
+    X = np.concatenate([[[0, 0, -1.0], [0, 0, 1.0]], np.stack([np.cos(t), np.sin(t), 0.1 * np.sin(3 * t)], 1)])
+    r = 2 + np.arange(n)
+    el = np.stack([np.zeros(n, int), r, 2 + (np.arange(n) + 1) % n, np.ones(n, int)], 1)
+    return X, el
+
+
+def mesh(kind):
+    from fea_b200.meshes import tet_block
+    rng = np.random.default_rng(1)
+    if kind == "fan":
+        X, el = fan(120)
+    else:
+        X, el = tet_block(0, dims=kind)
+        X = X + rng.uniform(-0.05, 0.05, X.shape) / max(kind)
+        perm = rng.permutation(len(X))
+        inv = np.empty(len(X), np.int64)
+        inv[perm] = np.arange(len(X))
+        X, el = X[perm], inv[el]
+    return X, el
+
+
+@gpu
+@pytest.mark.parametrize("kind", [(1, 1, 1), (2, 1, 1), (5, 4, 3), (9, 8, 7), "fan"])
+@pytest.mark.parametrize("repeat", [False, True])
+def test_lists_match_rank_rounds(kind, repeat):
+    from fea_b200 import DevicePlan
+    from fea_b200 import _lib as L
+    X, el = mesh(kind)
+    N = len(X)
+    if repeat:
+        el = np.concatenate([el, el[-1:]])        # a doubled element
+    mask = np.full(N, 7, np.uint8)
+    mask[N // 2], mask[N // 3], mask[-1] = 0, 5, 2
+    P = DevicePlan(X, mask, [("C3D4", el)])
+    g = P.groups[0]
+    gc = torch.from_numpy(np.random.default_rng(2).normal(0, 5e-3 / (1 if kind == "fan" else max(kind)), P.ndof)).cuda()
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    old = L.Group()
+    C.memmove(C.byref(old), C.byref(g.desc), C.sizeof(L.Group))
+    old.clist_dev = None
+    for acc in (0, 1):
+        for with_R in (True, False):
+            for with_e in (False, True):
+                out = []
+                for d in (old, g.desc):
+                    pad = torch.full((P.nnz + 64,), 0.5, dtype=torch.float64, device="cuda")
+                    R = torch.full((P.ndof + 64,), 0.25, dtype=torch.float64, device="cuda")
+                    eR = torch.zeros(12 * g.ne, dtype=torch.float64, device="cuda")
+                    L.check(L.fea_assemble_volume(C.byref(P.nodes), C.byref(d), 1.0, 30.0, ptr(gc), ptr(pad),
+                                                  ptr(R) if with_R else None, ptr(eR) if with_e else None, acc, None, 0,
+                                                  st), "tet")
+                    assert bool((pad[P.nnz:] == 0.5).all()) and bool((R[P.ndof:] == 0.25).all())
+                    out.append((pad, R, eR))
+                for a, b in zip(*out):
+                    assert float((a - b).abs().max()) <= TOL * max(1.0, float(a.abs().max()))
+
+
+def test_lists_of_the_host_plan():
+    """Every column's list holds, in incidence order, the blocks of the
+    incident elements that fall on its node."""
+    from fea_b200 import _lib as L
+    from fea_b200.plan import HostPlan
+    X, el = mesh((3, 2, 2))
+    el[0, 3] = el[0, 2]                           # an element that repeats a node (its values are 0/0)
+    N = len(X)
+    mask = np.full(N, 7, np.uint8)
+    mask[3], mask[5], mask[8] = 0, 6, 1
+    hp = HostPlan(N, mask, [(L.FEA_C3D4, el)], [])
+    crec, cptr = hp.array(L.FEA_A_G_CREC), hp.array(L.FEA_A_G_CRECPTR)
+    clist, nodeinc, inc = hp.array(L.FEA_A_G_CLIST), hp.array(L.G_BASE + L.A_NODEINC), hp.array(L.G_BASE + L.A_INC)
+    adjptr, adjcol, adjoff = hp.array(L.FEA_A_ADJPTR), hp.array(L.FEA_A_ADJCOL), hp.array(L.FEA_A_ADJOFF)
+    for n in range(N):
+        if mask[n] == 0:
+            continue
+        nb = [n] + [c for c in adjcol[adjptr[n]:adjptr[n + 1]] if c != n]
+        assert cptr[n + 1] - cptr[n] == len(nb)
+        for u, c in enumerate(nb):
+            want = [39 * r + 9 * b for r, q in enumerate(range(nodeinc[n], nodeinc[n + 1]))
+                    for b in range(4) if el[inc[q] >> 4, b] == c]
+            x, y = (int(v) for v in crec[2 * (cptr[n] + u):2 * (cptr[n] + u) + 2])
+            p = adjptr[n] + list(adjcol[adjptr[n]:adjptr[n + 1]]).index(c)
+            assert (x & 0xffff, x >> 16) == (adjoff[p], mask[c])
+            s, k = y & 0x7ff, y >> 11
+            assert list(clist[4 * nodeinc[n] + s:4 * nodeinc[n] + s + k]) == want
+    # tiles of at most 128 incidences
+    cl, tp = hp.array(L.G_BASE + L.A_CHUNKLIST), hp.array(L.FEA_A_G_TILEPTR)
+    assert tp[0] == 0 and tp[-1] == len(cl) and np.all(np.diff(tp) > 0) and len(tp) > 3
+    assert np.all(np.diff([nodeinc[n] for n in cl[tp[:-1]]] + [nodeinc[-1]]) <= 128)
