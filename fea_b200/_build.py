@@ -52,7 +52,7 @@ def _compile(src, verbose):
 
 def build(verbose=False, force=False):
     srcs = CU_SOURCES + CPP_SOURCES
-    deps = [os.path.join(CSRC, s) for s in srcs] + [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "hexlane.cuh"),
+    deps = [os.path.join(CSRC, s) for s in srcs] + [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "hexlane.cuh"), os.path.join(CSRC, "pcg_persist.cuh"),
                                                    os.path.join(ROOT, "include", "fea_b200.h")]
     if not force and os.path.exists(LIB) and all(os.path.getmtime(LIB) >= os.path.getmtime(d) for d in deps):
         return LIB

@@ -38,7 +38,13 @@ constexpr int PCG_WARPS = PCG_TPB / 32;
 constexpr int PCG_GRID = 148 * 8;   // fixed grid: bounds the partial count
 
 // device-side solver state (doubles, in the work buffer)
-enum { S_RZ = 0, S_RZ0, S_ALPHA, S_BETA, S_DONE, S_ITER, S_STATUS, S_PQ, S_COUNT, S_LEN = 16 };
+enum { S_RZ = 0, S_RZ0, S_ALPHA, S_BETA, S_DONE, S_ITER, S_STATUS, S_PQ, S_COUNT, S_NEED, S_FAIL, S_LEN = 16 };
+
+}  // namespace fea
+
+#include "pcg_persist.cuh"
+
+namespace fea {
 
 template <class V>
 struct CsrOp {
@@ -614,13 +620,14 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcg_p(int64_t n, X* __restrict__ p,
   }
 }
 
-// setup (dinv given): r = b - Ax (Ax in r on entry), z = dinv r, p = z,
+// setup (dinv given): r = b - Ax (Ax in r on entry), z = dinv r, p = z (p
+// NULL: z holds the pairs (epoch 0, z) of k_pcg_persist and q its p, 0),
 // partial r.z and b.dinv.b; last block initialises the state.
 template <class X>
 __global__ void __launch_bounds__(PCG_TPB) k_pcg_setup(int64_t n, const double* __restrict__ b, X* __restrict__ r,
                                                        X* __restrict__ z, X* __restrict__ p,
                                                        const double* __restrict__ dinv, double* st, double* part,
-                                                       unsigned* counter) {
+                                                       unsigned* counter, X* __restrict__ q = nullptr) {
   __shared__ double sh[PCG_WARPS];
   double c_rz = 0.0, c_bb = 0.0;
   for (int64_t i = (int64_t)blockIdx.x * PCG_TPB + threadIdx.x; i < n; i += (int64_t)gridDim.x * PCG_TPB) {
@@ -628,8 +635,14 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcg_setup(int64_t n, const double* 
     double ri = b[i] - (double)r[i];
     r[i] = (X)ri;
     double zi = ri * di;
-    z[i] = (X)zi;
-    p[i] = (X)zi;
+    if (p) {
+      z[i] = (X)zi;
+      p[i] = (X)zi;
+    } else {
+      z[2 * i] = (X)0;
+      z[2 * i + 1] = (X)zi;
+      q[i] = (X)0;
+    }
     c_rz += ri * zi;
     c_bb += b[i] * b[i] * di;
   }
@@ -647,6 +660,9 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcg_setup(int64_t n, const double* 
       st[S_RZ0] = bb;
       st[S_ITER] = 0.0;
       st[S_STATUS] = 0.0;
+      st[S_BETA] = 0.0;
+      st[S_COUNT] = 0.0;
+      st[S_FAIL] = 0.0;
       // a zero right-hand side or an exact initial guess needs no iteration
       st[S_DONE] = (bb == 0.0 || rz == 0.0) ? 1.0 : 0.0;
       if (bb == 0.0) st[S_RZ0] = 1.0;
@@ -858,6 +874,83 @@ static int pcg_core(const Op& A, int64_t n, const double* b, X* x, X* r, X* z, X
     }
     if (cudaError_t e = cudaGetLastError()) return (int)e;
     it_done += batch;
+  }
+  if (iters) *iters = (int)host[S_ITER];
+  if (relres) *relres = host[S_RZ] / host[S_RZ0];
+  return (int)host[S_STATUS];
+}
+
+static int smem_optin() {
+  int dev = 0, v = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return v;
+}
+
+// CTAs of k_pcg_persist: one per SM, fewer when a CTA would own less than
+// PP_ROWS rows (a smaller grid sums faster).
+#ifndef FEA_PP_ROWS
+#define FEA_PP_ROWS 72
+#endif
+static unsigned persist_grid(int64_t n) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::min(sms, PP_MAXG), n / FEA_PP_ROWS));
+}
+
+// PCG on a matrix that fits the shared memory of the grid's CTAs; *fits = false
+// (and nothing done) when it does not: the largest share is known once
+// k_persist_plan has run, which systems that cannot fit are spared.
+static int pcg_persist(const NodeOp<double>& A, int64_t nnz, const double* b, double* x, double tol, int max_iter,
+                       int check_every, const PcgWork& W, bool* fits, int* iters, double* relres, cudaStream_t s) {
+  *fits = false;
+  const int64_t n = A.n;
+  const unsigned G = persist_grid(n);
+  const int64_t lim = smem_optin() - (int64_t)sizeof(PersistShared) - 64;
+  const int64_t bitmap = 4 * ((n + 31) / 32);
+  if (8 * nnz / G > lim || bitmap > lim) return 0;
+  ulonglong2* slots = reinterpret_cast<ulonglong2*>(((uintptr_t)W.part + 15) & ~(uintptr_t)15);
+  PersistArgs P{A.vbase, A.rowlen, A.dbase, A.mask, A.idx, A.val, A.n_nodes, n, x, W.r, W.q, W.dinv,
+                reinterpret_cast<ulonglong2*>(W.z), W.st, slots, reinterpret_cast<unsigned*>(slots + 2 * G),
+                reinterpret_cast<int64_t*>(slots + 2 * G + 1), tol,
+                max_iter, 0, 0};
+  spmv(A, (const double*)x, W.r, nullptr, nullptr, nullptr, 0, s);       // r = A x
+  k_pcg_setup<double><<<vec_grid<double>(n), PCG_TPB, 0, s>>>(n, b, W.r, W.z, nullptr, W.dinv, W.st, W.part, W.counter,
+                                                             W.q);
+  cudaMemsetAsync(slots, 0, sizeof(ulonglong2) * (2 * G + 1), s);
+  cudaMemsetAsync(W.st + S_NEED, 0, sizeof(double), s);
+  if (cudaError_t e = cudaFuncSetAttribute(k_persist_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitmap))
+    return (int)e;
+  k_persist_plan<<<G, PP_TPB, (size_t)bitmap, s>>>(P);
+  count_launch(2);
+  if (cudaError_t e = cudaGetLastError()) return (int)e;
+  // iterations per launch: at least the caller's check_every, about a
+  // millisecond or two (the kernel itself stops at convergence)
+  const int64_t per = ((int64_t)1 << 32) / (8 * nnz + 1);
+  const int ce = (int)std::max<int64_t>(std::max(1, check_every), std::min<int64_t>(512, per));
+  double host[S_LEN];
+  int it_done = 0;
+  while (true) {
+    cudaMemcpyAsync(host, W.st, sizeof(host), cudaMemcpyDeviceToHost, s);
+    if (cudaError_t e = cudaStreamSynchronize(s)) return (int)e;
+    if (!*fits) {
+      unsigned long long need;
+      std::memcpy(&need, host + S_NEED, sizeof(need));
+      if (need > (unsigned long long)lim) return 0;
+      *fits = true;
+      P.smem = (unsigned)need;
+      if (cudaError_t e = cudaFuncSetAttribute(k_pcg_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need))
+        return (int)e;
+    }
+    if (host[S_FAIL] != 0.0) return FEA_ETIMEOUT;
+    if (host[S_DONE] != 0.0 || it_done >= max_iter) break;
+    P.iters = std::min(ce, max_iter - it_done);
+    void* args[] = {&P};
+    if (cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_pcg_persist, dim3(G), dim3(PP_TPB), args, P.smem, s))
+      return (int)e;
+    count_launch();
+    it_done += P.iters;
   }
   if (iters) *iters = (int)host[S_ITER];
   if (relres) *relres = host[S_RZ] / host[S_RZ0];
@@ -1516,7 +1609,18 @@ extern "C" int fea_pcg_solve_nodes(const fea_nodes_t* N, const int32_t* ix, cons
   if (iters) *iters = 0;
   if (relres) *relres = 0.0;
   if (n == 0) return FEA_OK;
-  return pcg_fp64(node_op<double>(N, ix, v), n, b, x, tol, max_iter, check_every, 1, work, iters, relres, s);
+  const NodeOp<double> A = node_op<double>(N, ix, v);
+  if (((uintptr_t)work & 15) == 0) {             // (the pairs of k_pcg_persist are 16-byte aligned)
+    const PcgWork W = carve(work, n);
+    cudaMemsetAsync(W.counter, 0, 2 * sizeof(unsigned), s);
+    diag_inv(A, W.dinv, 1, s);
+    bool fits = false;
+    int it = 0;
+    const int r = pcg_persist(A, N->nnz, b, x, tol, max_iter, check_every, W, &fits, &it, relres, s);
+    if (iters) *iters = it;
+    if (fits || r != 0) return r;
+  }
+  return pcg_fp64(A, n, b, x, tol, max_iter, check_every, 1, work, iters, relres, s);
 }
 
 extern "C" int fea_pcg_solve_mixed(int64_t n, const int64_t* ip, const int32_t* ix, const double* v,

@@ -50,6 +50,7 @@ extern "C" {
 #define FEA_EBREAKDOWN -7  /* PCG breakdown (p.Ap <= 0 or non-finite) */
 #define FEA_ETOOBIG -8     /* size beyond a fixed limit: of an allocation-free entry point, or a
                               group of more than FEA_PLAN_MAX_ELEMS elements or faces */
+#define FEA_ETIMEOUT -9    /* a bounded wait between the blocks of one launch ran out (PCG) */
 
 /* C3D4 assembly: incidences per tile (threads per CTA), and doubles per
  * incidence in the kernel's shared memory (4 blocks of 9, residual 3) */
