@@ -9,8 +9,9 @@
 // M = |diag K| (x = D^-1 x~, r = D r~), so this file runs PCG directly and
 // evaluates the same stop test as (r.M^-1 r) / (b.M^-1 b).
 //
-// One iteration = 3 kernels: (1) q = K p fused with p.q, (2) x, r, z update
-// fused with r.z, (3) p update.  Scalars (alpha, beta, r.z, status) stay on
+// One iteration = 2 kernels: (1) q = K p fused with p = z + beta p and p.q, (2)
+// x, r, z update fused with r.z; or, for systems that fit the shared memory,
+// many iterations in one launch (pcg_persist.cuh).  Scalars (alpha, beta, r.z, status) stay on
 // the device; every dot product is a fixed-order two-level sum (per-block
 // partials over a fixed grid, summed by the last block to finish), so
 // results are bitwise reproducible.  The host reads the status every
@@ -66,6 +67,69 @@ struct NodeOp {
   int64_t n_nodes;
   int64_t n;      // rows (free DOFs)
 };
+
+// The vector an SpMV multiplies: a plain one, or p = z + beta p_old formed from
+// the pairs (z, p_old) of the rows as it is gathered (one kernel less per
+// iteration than with p in an array of its own; the update kernel writes the
+// pairs back).
+template <class X>
+struct PlainVec {
+  const X* __restrict__ x;
+  __device__ __forceinline__ void init() {}
+  __device__ __forceinline__ X operator()(int64_t j) const { return x[j]; }
+};
+template <class X>
+struct PairVec;
+template <>
+struct PairVec<double> {
+  const double2* __restrict__ zp;
+  const double* st;
+  double beta;
+  __device__ __forceinline__ void init() { beta = st[S_BETA]; }
+  __device__ __forceinline__ double operator()(int64_t j) const {
+    return of(zp[j]);
+  }
+  __device__ __forceinline__ double of(double2 t) const { return fma(beta, t.y, t.x); }
+};
+template <>
+struct PairVec<float> {
+  const float2* __restrict__ zp;
+  const double* st;
+  float bh, bl;                      // beta to 48 bits
+  __device__ __forceinline__ void init() {
+    const double b = st[S_BETA];
+    bh = (float)b;
+    bl = (float)(b - (double)bh);
+  }
+  __device__ __forceinline__ float operator()(int64_t j) const {
+    return of(zp[j]);
+  }
+  __device__ __forceinline__ float of(float2 t) const { return fmaf(bh, t.y, fmaf(bl, t.y, t.x)); }
+};
+template <class X>
+struct PairOf;
+template <>
+struct PairOf<double> { typedef double2 type; };
+template <>
+struct PairOf<float> { typedef float2 type; };
+
+// Programmatic dependent launch: a kernel's start overlaps the end of the one
+// before it; grid_wait() holds it until that one's results are there.
+__device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... Q>
+static void launch_after(void (*k)(P...), unsigned grid, unsigned threads, cudaStream_t s, Q... q) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(threads);
+  c.stream = s;
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = a;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, P(q)...);
+}
 
 // block sum: warp shuffles, then the 8 warp sums in fixed order
 __device__ __forceinline__ double block_sum_w(double v, double* sh) {
@@ -132,10 +196,13 @@ __device__ __forceinline__ void finish_pq(double contrib, double* st, double* pa
 
 // ---- CSR operator: LANES threads per row, warp-uniform loop ----------------
 // y = A x ; mode 1: also p.q partials and the alpha epilogue
-template <int LANES, class V, class X>
-__global__ void __launch_bounds__(PCG_TPB) k_spmv_csr(CsrOp<V> A, const X* __restrict__ x, X* __restrict__ y,
+template <int LANES, class V, class X, class Vec>
+__global__ void __launch_bounds__(PCG_TPB) k_spmv_csr(CsrOp<V> A, Vec x, X* __restrict__ y,
                                                       double* st, double* part, unsigned* counter, int mode) {
+  grid_next();
+  grid_wait();
   if (mode == 1 && st[S_DONE] != 0.0) return;
+  x.init();
   constexpr int RPW = 32 / LANES;                 // rows per warp
   const int lane = threadIdx.x % LANES;
   const int warp = threadIdx.x >> 5;
@@ -147,23 +214,23 @@ __global__ void __launch_bounds__(PCG_TPB) k_spmv_csr(CsrOp<V> A, const X* __res
     double s = 0.0;
     if (row < A.n) {
       const int64_t b = A.ptr[row], e = A.ptr[row + 1];
-      for (int64_t i = b + lane; i < e; i += LANES) s += (double)A.val[i] * (double)x[A.idx[i]];
+      for (int64_t i = b + lane; i < e; i += LANES) s += (double)A.val[i] * (double)x(A.idx[i]);
     }
 #pragma unroll
     for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LANES);
     if (row < A.n && lane == 0) {
       y[row] = (X)s;
-      contrib += s * (double)x[row];
+      contrib += s * (double)x(row);
     }
   }
   if (mode == 1) finish_pq(contrib, st, part, counter);
 }
 
 // ---- node operator: one warp per node row block ------------------------------
-template <class V, class X>
-__global__ void __launch_bounds__(PCG_TPB) k_spmv_node(NodeOp<V> A, const X* __restrict__ x, X* __restrict__ y,
+template <class V, class X, class Vec>
+__global__ void __launch_bounds__(PCG_TPB) k_spmv_node(NodeOp<V> A, Vec x, X* __restrict__ y,
                                                        double* st, double* part, unsigned* counter, int mode) {
-  if (mode == 1 && st[S_DONE] != 0.0) return;
+  grid_next();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int64_t step = (int64_t)gridDim.x * PCG_WARPS;
@@ -183,6 +250,9 @@ __global__ void __launch_bounds__(PCG_TPB) k_spmv_node(NodeOp<V> A, const X* __r
 #pragma unroll
     for (int k = 0; k < 3; ++k) jn[k] = lane + 32 * k < L ? __ldg(A.idx + vb + lane + 32 * k) : 0;
   }
+  grid_wait();                                       // (the matrix does not depend on the kernel before)
+  if (mode == 1 && st[S_DONE] != 0.0) return;
+  x.init();
   while (nd < A.n_nodes) {
     const int64_t nx = nd + step;
     unsigned m2 = 0;
@@ -218,7 +288,7 @@ __global__ void __launch_bounds__(PCG_TPB) k_spmv_node(NodeOp<V> A, const X* __r
           }
         double xv[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) xv[k] = h[k] ? (double)x[j[k]] : 0.0;
+        for (int k = 0; k < 3; ++k) xv[k] = h[k] ? (double)x(j[k]) : 0.0;
         s0 += va[0][0] * xv[0] + va[0][1] * xv[1] + va[0][2] * xv[2];
         s1 += va[1][0] * xv[0] + va[1][1] * xv[1] + va[1][2] * xv[2];
         s2 += va[2][0] * xv[0] + va[2][1] * xv[1] + va[2][2] * xv[2];
@@ -238,9 +308,9 @@ __global__ void __launch_bounds__(PCG_TPB) k_spmv_node(NodeOp<V> A, const X* __r
       if (lane == 0) {
         const int64_t r = A.dbase[nd];
         y[r] = (X)s0;
-        contrib += s0 * (double)x[r];
-        if (f > 1) { y[r + 1] = (X)s1; contrib += s1 * (double)x[r + 1]; }
-        if (f > 2) { y[r + 2] = (X)s2; contrib += s2 * (double)x[r + 2]; }
+        contrib += s0 * (double)x(r);
+        if (f > 1) { y[r + 1] = (X)s1; contrib += s1 * (double)x(r + 1); }
+        if (f > 2) { y[r + 2] = (X)s2; contrib += s2 * (double)x(r + 2); }
       }
     }
     nd = nx;
@@ -260,10 +330,13 @@ __global__ void __launch_bounds__(PCG_TPB) k_spmv_node(NodeOp<V> A, const X* __r
 // passes (CPL = 6) need 77 registers, 3 CTAs per SM, and ran the FP32
 // iteration 0.237 ms against 0.134 ms at 64^3.  Loops and shuffles
 // warp-uniform.
-template <int LPN, int CPL, class V, class X>
-__global__ void __launch_bounds__(PCG_TPB) k_spmv_node_sub(NodeOp<V> A, const X* __restrict__ x, X* __restrict__ y,
+template <int LPN, int CPL, class V, class X, class Vec>
+__global__ void __launch_bounds__(PCG_TPB) k_spmv_node_sub(NodeOp<V> A, Vec x, X* __restrict__ y,
                                                            double* st, double* part, unsigned* counter, int mode) {
+  grid_next();
+  grid_wait();
   if (mode == 1 && st[S_DONE] != 0.0) return;
+  x.init();
   constexpr int NPW = 32 / LPN;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -324,7 +397,7 @@ __global__ void __launch_bounds__(PCG_TPB) k_spmv_node_sub(NodeOp<V> A, const X*
         }
       double xv[CPL];
 #pragma unroll
-      for (int k = 0; k < CPL; ++k) xv[k] = h[k] ? (double)x[j[k]] : 0.0;
+      for (int k = 0; k < CPL; ++k) xv[k] = h[k] ? (double)x(j[k]) : 0.0;
       if constexpr (CPL == 3) {
         s0 += va[0][0] * xv[0] + va[0][1] * xv[1] + va[0][2] * xv[2];
         s1 += va[1][0] * xv[0] + va[1][1] * xv[1] + va[1][2] * xv[2];
@@ -351,7 +424,7 @@ __global__ void __launch_bounds__(PCG_TPB) k_spmv_node_sub(NodeOp<V> A, const X*
       const int64_t r = db + hl;
       const double sr = hl == 0 ? s0 : (hl == 1 ? s1 : s2);
       y[r] = (X)sr;
-      contrib += sr * (double)x[r];
+      contrib += sr * (double)x(r);
     }
     nd = nx;
     m = m2;
@@ -383,10 +456,13 @@ struct NodeOp32q {
 #ifndef FEA_F32Q_LPN
 #define FEA_F32Q_LPN 8
 #endif
-template <int LPN, class X>
-__global__ void __launch_bounds__(PCG_TPB, 4) k_spmv_node32q(NodeOp32q A, const X* __restrict__ x, X* __restrict__ y,
+template <int LPN, class X, class Vec>
+__global__ void __launch_bounds__(PCG_TPB, 4) k_spmv_node32q(NodeOp32q A, Vec x, X* __restrict__ y,
                                                              double* st, double* part, unsigned* counter, int mode) {
+  grid_next();
+  grid_wait();
   if (mode == 1 && st[S_DONE] != 0.0) return;
+  x.init();
   constexpr int NPW = 32 / LPN;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -435,10 +511,10 @@ __global__ void __launch_bounds__(PCG_TPB, 4) k_spmv_node32q(NodeOp32q A, const 
       const float4 v2 = (h && f > 2) ? __ldcs(reinterpret_cast<const float4*>(A.vals + qb + 2 * L4 + q)) : z4;
       float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f;
       if (h) {
-        x0 = (float)x[c.x];
-        x1 = (float)x[c.y];
-        x2 = (float)x[c.z];
-        x3 = (float)x[c.w];
+        x0 = (float)x(c.x);
+        x1 = (float)x(c.y);
+        x2 = (float)x(c.z);
+        x3 = (float)x(c.w);
       }
       s0 += v0.x * x0 + v0.y * x1 + v0.z * x2 + v0.w * x3;
       s1 += v1.x * x0 + v1.y * x1 + v1.z * x2 + v1.w * x3;
@@ -454,7 +530,7 @@ __global__ void __launch_bounds__(PCG_TPB, 4) k_spmv_node32q(NodeOp32q A, const 
       const int64_t r = db + hl;
       const double sr = (double)(hl == 0 ? s0 : (hl == 1 ? s1 : s2));
       y[r] = (X)sr;
-      contrib += sr * (double)x[r];
+      contrib += sr * (double)x(r);
     }
     nd = nx;
     m = m2;
@@ -528,26 +604,34 @@ __global__ void k_dinv_csr(CsrOp<V> A, double* __restrict__ dinv, int identity) 
   }
 }
 
-// x += alpha p; r -= alpha q; z = r / |d|; partial r.z; last block: beta, stop test.
+// x += alpha p; r -= alpha q; z = r / |d|; (z, p) back; partial r.z; last block: beta,
+// stop test.
 // Each thread takes PCG_VU rows a grid stride apart and issues all their
 // loads before any arithmetic (one resident wave covers the vector in one
 // pass up to PCG_VU x 303k rows), so the loads of a thread overlap instead
 // of paying one round trip per row.
 constexpr int PCG_VU = 4;
 
-template <class X>
+template <class X, bool PAIRS>
 __global__ void __launch_bounds__(PCG_TPB) k_pcg_update(int64_t n, X* __restrict__ x, X* __restrict__ r,
-                                                        X* __restrict__ z, const X* __restrict__ p,
+                                                        typename PairOf<X>::type* __restrict__ zp,
                                                         const X* __restrict__ q, const double* __restrict__ dinv,
                                                         double* st, double* part, unsigned* counter, double tol,
                                                         int max_iter) {
   __shared__ double sh[PCG_WARPS];
+  grid_next();
+  grid_wait();
   if (st[S_DONE] != 0.0) return;
   const double alpha = st[S_ALPHA];
+  PairVec<X> pv;
+  pv.st = st;
+  pv.init();
+  X *z = reinterpret_cast<X*>(zp), *pa = z + n;    // (not PAIRS: z, then p)
   double contrib = 0.0;
   const int64_t stride = (int64_t)gridDim.x * PCG_TPB;
   for (int64_t i0 = (int64_t)blockIdx.x * PCG_TPB + threadIdx.x; i0 < n; i0 += PCG_VU * stride) {
-    X xv[PCG_VU], rv[PCG_VU], pv[PCG_VU], qv[PCG_VU];
+    X xv[PCG_VU], rv[PCG_VU], qv[PCG_VU];
+    typename PairOf<X>::type tv[PCG_VU];
     double dv[PCG_VU];
 #pragma unroll
     for (int u = 0; u < PCG_VU; ++u) {
@@ -555,7 +639,8 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcg_update(int64_t n, X* __restrict
       if (i < n) {
         xv[u] = x[i];
         rv[u] = r[i];
-        pv[u] = p[i];
+        if (PAIRS) tv[u] = zp[i];
+        else tv[u].y = pa[i];
         qv[u] = q[i];
         dv[u] = dinv[i];
       }
@@ -564,11 +649,19 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcg_update(int64_t n, X* __restrict
     for (int u = 0; u < PCG_VU; ++u) {
       const int64_t i = i0 + u * stride;
       if (i < n) {
-        x[i] = (X)((double)xv[u] + alpha * (double)pv[u]);
+        const X p = PAIRS ? pv.of(tv[u]) : tv[u].y;   // the p that the SpMV multiplied
+        x[i] = (X)((double)xv[u] + alpha * (double)p);
         const double ri = (double)rv[u] - alpha * (double)qv[u];
         r[i] = (X)ri;
         const double zi = ri * dv[u];
-        z[i] = (X)zi;
+        if (PAIRS) {
+          typename PairOf<X>::type t;
+          t.x = (X)zi;
+          t.y = p;
+          zp[i] = t;
+        } else {
+          z[i] = (X)zi;
+        }
         contrib += ri * zi;
       }
     }
@@ -596,9 +689,12 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcg_update(int64_t n, X* __restrict
   }
 }
 
+// p = z + beta p of large systems (z, p: arrays of their own)
 template <class X>
 __global__ void __launch_bounds__(PCG_TPB) k_pcg_p(int64_t n, X* __restrict__ p, const X* __restrict__ z,
                                                    const double* st) {
+  grid_next();
+  grid_wait();
   if (st[S_DONE] != 0.0) return;
   const double beta = st[S_BETA];
   const int64_t stride = (int64_t)gridDim.x * PCG_TPB;
@@ -620,28 +716,33 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcg_p(int64_t n, X* __restrict__ p,
   }
 }
 
-// setup (dinv given): r = b - Ax (Ax in r on entry), z = dinv r, p = z (p
-// NULL: z holds the pairs (epoch 0, z) of k_pcg_persist and q its p, 0),
+// setup (dinv given): r = b - Ax (Ax in r on entry), z = dinv r, beta = 0 and,
+// by form, the pairs (z, 0) (FORM_PAIRS), z and p = 0 in arrays of their own
+// (FORM_ARRAYS), or k_pcg_persist's (epoch 0, z) and p0 = 0 (FORM_TAGS);
 // partial r.z and b.dinv.b; last block initialises the state.
+enum { FORM_PAIRS, FORM_ARRAYS, FORM_TAGS };
 template <class X>
 __global__ void __launch_bounds__(PCG_TPB) k_pcg_setup(int64_t n, const double* __restrict__ b, X* __restrict__ r,
-                                                       X* __restrict__ z, X* __restrict__ p,
+                                                       typename PairOf<X>::type* __restrict__ zp,
                                                        const double* __restrict__ dinv, double* st, double* part,
-                                                       unsigned* counter, X* __restrict__ q = nullptr) {
+                                                       unsigned* counter, int form, X* __restrict__ p0) {
   __shared__ double sh[PCG_WARPS];
+  X* za = reinterpret_cast<X*>(zp);
   double c_rz = 0.0, c_bb = 0.0;
   for (int64_t i = (int64_t)blockIdx.x * PCG_TPB + threadIdx.x; i < n; i += (int64_t)gridDim.x * PCG_TPB) {
     const double di = dinv[i];
     double ri = b[i] - (double)r[i];
     r[i] = (X)ri;
     double zi = ri * di;
-    if (p) {
-      z[i] = (X)zi;
-      p[i] = (X)zi;
+    if (form == FORM_ARRAYS) {
+      za[i] = (X)zi;
+      za[n + i] = (X)0;
     } else {
-      z[2 * i] = (X)0;
-      z[2 * i + 1] = (X)zi;
-      q[i] = (X)0;
+      typename PairOf<X>::type t;
+      t.x = form == FORM_TAGS ? (X)0 : (X)zi;
+      t.y = form == FORM_TAGS ? (X)zi : (X)0;
+      zp[i] = t;
+      if (form == FORM_TAGS) p0[i] = (X)0;
     }
     c_rz += ri * zi;
     c_bb += b[i] * b[i] * di;
@@ -683,14 +784,14 @@ __global__ void k_axpy_f32(int64_t n, double* __restrict__ x, const float* __res
 
 // Residual replacement of the mixed solver (after x64 += x32, x32 = 0):
 // r64 = b - A x64 (A x64 in r64 on entry), r32 = float(r64), z32 =
-// float(r32 dinv), and in the last block: the true stop test
+// float(r32 dinv) into the pairs, and in the last block: the true stop test
 // (r64.D^-1 r64)/(b.D^-1 b) into st64, rho' = r32.z32 and beta' = rho' beta /
 // rho (the FP32 recurrence continues with the true residual and the same
 // search direction), and the FP32 done flag cleared unless the true residual
 // has converged.
 __global__ void __launch_bounds__(PCG_TPB) k_mixed_replace(int64_t n, const double* __restrict__ b,
                                                            double* __restrict__ r64, const double* __restrict__ dinv,
-                                                           float* __restrict__ r32, float* __restrict__ z32,
+                                                           float* __restrict__ r32, float2* __restrict__ zp32, int form,
                                                            double* st64, double* st32, double* part,
                                                            unsigned* counter, double tol) {
   __shared__ double sh[PCG_WARPS];
@@ -701,8 +802,8 @@ __global__ void __launch_bounds__(PCG_TPB) k_mixed_replace(int64_t n, const doub
     const float rf = (float)ri;
     r32[i] = rf;
     const double zi = (double)rf * dinv[i];
-    const float zf = (float)zi;
-    z32[i] = zf;
+    if (form == FORM_PAIRS) zp32[i].x = (float)zi;   // (p_old stays)
+    else reinterpret_cast<float*>(zp32)[i] = (float)zi;
     c_rr += ri * ri * dinv[i];
     c_rz += (double)rf * zi;
   }
@@ -768,40 +869,42 @@ static unsigned fixed_grid(int64_t units, int per_block) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(g, PCG_GRID));
 }
 
-template <class V, class X>
-static void spmv(const CsrOp<V>& A, const X* x, X* y, double* st, double* part, unsigned* counter, int mode,
-                 cudaStream_t s) {
+// y = A x on a plain vector (mode 0) or on the pairs (mode 1, with p.q and the
+// alpha epilogue); one after the other on the stream
+template <class V, class X, class Vec>
+static void spmv_on(const CsrOp<V>& A, Vec x, X* y, double* st, double* part, unsigned* counter, int mode,
+                    cudaStream_t s) {
   const int L = lanes_for(A.n, A.nnz);
-  const int rpb = PCG_TPB / L;
-  if (L == 32) k_spmv_csr<32, V, X><<<occ_grid(k_spmv_csr<32, V, X>, A.n, rpb), PCG_TPB, 0, s>>>(A, x, y, st, part,
-                                                                                            counter, mode);
-  else if (L == 16) k_spmv_csr<16, V, X><<<occ_grid(k_spmv_csr<16, V, X>, A.n, rpb), PCG_TPB, 0, s>>>(A, x, y, st,
-                                                                                                 part, counter, mode);
-  else k_spmv_csr<8, V, X><<<occ_grid(k_spmv_csr<8, V, X>, A.n, rpb), PCG_TPB, 0, s>>>(A, x, y, st, part, counter,
-                                                                                  mode);
+  auto k = L == 32 ? k_spmv_csr<32, V, X, Vec> : (L == 16 ? k_spmv_csr<16, V, X, Vec> : k_spmv_csr<8, V, X, Vec>);
+  launch_after(k, occ_grid(k, A.n, PCG_TPB / L), PCG_TPB, s, A, x, y, st, part, counter, mode);
   count_launch();
 }
 
-template <class V, class X>
-static void spmv(const NodeOp<V>& A, const X* x, X* y, double* st, double* part, unsigned* counter, int mode,
-                 cudaStream_t s) {
-  if (sizeof(V) == 4) {
-    k_spmv_node_sub<16, 3, V, X><<<occ_grid(k_spmv_node_sub<16, 3, V, X>, A.n_nodes, 2 * PCG_WARPS), PCG_TPB, 0, s>>>(
-        A, x, y, st, part, counter, mode);
+template <class V, class X, class Vec>
+static void spmv_on(const NodeOp<V>& A, Vec x, X* y, double* st, double* part, unsigned* counter, int mode,
+                    cudaStream_t s) {
+  if constexpr (sizeof(V) == 4) {
+    auto k = k_spmv_node_sub<16, 3, V, X, Vec>;
+    launch_after(k, occ_grid(k, A.n_nodes, 2 * PCG_WARPS), PCG_TPB, s, A, x, y, st, part, counter, mode);
   } else {
-    k_spmv_node<V, X><<<occ_grid(k_spmv_node<V, X>, A.n_nodes, PCG_WARPS), PCG_TPB, 0, s>>>(A, x, y, st, part,
-                                                                                          counter, mode);
+    auto k = k_spmv_node<V, X, Vec>;
+    launch_after(k, occ_grid(k, A.n_nodes, PCG_WARPS), PCG_TPB, s, A, x, y, st, part, counter, mode);
   }
   count_launch();
 }
 
-template <class X>
-static void spmv(const NodeOp32q& A, const X* x, X* y, double* st, double* part, unsigned* counter, int mode,
-                 cudaStream_t s) {
+template <class X, class Vec>
+static void spmv_on(const NodeOp32q& A, Vec x, X* y, double* st, double* part, unsigned* counter, int mode,
+                    cudaStream_t s) {
   constexpr int LPN = FEA_F32Q_LPN;
-  k_spmv_node32q<LPN, X><<<occ_grid(k_spmv_node32q<LPN, X>, A.n_nodes, PCG_WARPS * (32 / LPN)), PCG_TPB, 0, s>>>(
-      A, x, y, st, part, counter, mode);
+  auto k = k_spmv_node32q<LPN, X, Vec>;
+  launch_after(k, occ_grid(k, A.n_nodes, PCG_WARPS * (32 / LPN)), PCG_TPB, s, A, x, y, st, part, counter, mode);
   count_launch();
+}
+
+template <class Op, class X>
+static void spmv(const Op& A, const X* x, X* y, cudaStream_t s) {
+  spmv_on(A, PlainVec<X>{x}, y, (double*)nullptr, (double*)nullptr, (unsigned*)nullptr, 0, s);
 }
 
 template <class V>
@@ -819,17 +922,21 @@ static void diag_inv(const NodeOp<V>& A, double* dinv, int, cudaStream_t s) {
 template <class X>
 static unsigned vec_grid(int64_t n) {
   // the update kernel's wave sizes all three vector kernels (same partials)
-  return occ_grid(k_pcg_update<X>, n, PCG_TPB);
+  return occ_grid(k_pcg_update<X, true>, n, PCG_TPB);
 }
 
 static int64_t part_len(int64_t) { return 2 * PCG_GRID + 2; }
 
-// Work layout (doubles): st[S_LEN] | counter(2) | dinv[n] | r | z | p | q | part
+// Work layout (doubles): st[S_LEN] | counter(2) | dinv[n] | r | zp (2n) | q | part;
+// zp, q and part one double further when that puts the pairs on 16 bytes
+// (part has room for it)
 struct PcgWork {
   double* st;
   unsigned* counter;
   double* dinv;
-  double *r, *z, *p, *q;
+  double* r;
+  double2* zp;
+  double* q;
   double* part;
 };
 
@@ -839,38 +946,68 @@ static PcgWork carve(double* w, int64_t n) {
   W.counter = (unsigned*)(w + S_LEN);
   W.dinv = w + S_LEN + 2;
   W.r = W.dinv + n;
-  W.z = W.r + n;
-  W.p = W.z + n;
-  W.q = W.p + n;
+  double* z = W.r + n;
+  z += (uintptr_t)z >> 3 & 1;
+  W.zp = reinterpret_cast<double2*>(z);
+  W.q = z + 2 * n;
   W.part = W.q + n;
   return W;
 }
 
-// Run PCG iterations on (A, b) in precision X starting from x (in X), with
-// dinv given.  Returns status; *iters.  A64 computes the FP64 residual of
-// the initial guess (same operator in FP64 values).
+// Rows up to which p is formed in the gather (pairs); above, by a kernel of its
+// own: a pair is twice the gathered bytes, and once the rows' vectors crowd
+// the caches the SpMV loses more than the p kernel takes.  us per iteration,
+// pairs and arrays: FP64 38.8 and 39.9 at 202k rows (40^3 C3D8), 60.0 and 61.5
+// at 346k, 98.1 and 96.8 at 546k, 152 and 142 at 811k; FP32 27.4 and 29.1, 36.8
+// and 39.2, 57.7 and 62.9, 96.3 and 99.8 (larger ones not measured).
+constexpr int64_t PAIR_ROWS64 = 450000, PAIR_ROWS32 = 1000000;
+template <class X>
+static int form_for(int64_t n) {
+  return n <= (sizeof(X) == 8 ? PAIR_ROWS64 : PAIR_ROWS32) ? FORM_PAIRS : FORM_ARRAYS;
+}
+
+// One iteration: q = A p with p.q and alpha; x, r, z with r.z, beta and the stop test
 template <class Op, class X>
-static int pcg_core(const Op& A, int64_t n, const double* b, X* x, X* r, X* z, X* p, X* q, const double* dinv,
-                    double* st, unsigned* counter, double* part, double tol, int max_iter, int check_every,
-                    int* iters, double* relres, cudaStream_t s) {
-  spmv(A, (const X*)x, r, st, part, counter, 0, s);       // r = A x
-  const unsigned vg = vec_grid<X>(n);
-  k_pcg_setup<X><<<vg, PCG_TPB, 0, s>>>(n, b, r, z, p, dinv, st, part, counter);
+static void iterate(const Op& A, int64_t n, int form, unsigned vg, X* x, X* r, typename PairOf<X>::type* zp, X* q,
+                    const double* dinv, double* st, double* part, unsigned* counter, double tol, int max_iter,
+                    cudaStream_t s) {
+  if (form == FORM_PAIRS) {
+    PairVec<X> v;
+    v.zp = zp;
+    v.st = st;
+    spmv_on(A, v, q, st, part, counter, 1, s);
+    launch_after(k_pcg_update<X, true>, vg, PCG_TPB, s, n, x, r, zp, q, dinv, st, part, counter, tol, max_iter);
+  } else {
+    X* z = reinterpret_cast<X*>(zp);
+    launch_after(k_pcg_p<X>, vg, PCG_TPB, s, n, z + n, z, st);
+    spmv_on(A, PlainVec<X>{z + n}, q, st, part, counter, 1, s);
+    launch_after(k_pcg_update<X, false>, vg, PCG_TPB, s, n, x, r, zp, q, dinv, st, part, counter, tol, max_iter);
+    count_launch();
+  }
+  count_launch();
+}
+
+// FP64 PCG iterations on (A, b) from x with dinv given.
+// Returns the status; *iters.
+template <class Op>
+static int pcg_core(const Op& A, int64_t n, const double* b, double* x, const PcgWork& W, double tol, int max_iter,
+                    int check_every, int* iters, double* relres, cudaStream_t s) {
+  spmv(A, (const double*)x, W.r, s);                      // r = A x
+  const unsigned vg = vec_grid<double>(n);
+  const int form = form_for<double>(n);
+  k_pcg_setup<double><<<vg, PCG_TPB, 0, s>>>(n, b, W.r, W.zp, W.dinv, W.st, W.part, W.counter, form, nullptr);
   count_launch();
   if (cudaError_t e = cudaGetLastError()) return (int)e;
   double host[S_LEN];
   int it_done = 0;
   const int ce = std::max(1, check_every);
   while (true) {
-    cudaMemcpyAsync(host, st, sizeof(host), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(host, W.st, sizeof(host), cudaMemcpyDeviceToHost, s);
     if (cudaError_t e = cudaStreamSynchronize(s)) return (int)e;
     if (host[S_DONE] != 0.0 || it_done >= max_iter) break;
     const int batch = std::min(ce, max_iter - it_done);
     for (int k = 0; k < batch; ++k) {
-      spmv(A, (const X*)p, q, st, part, counter, 1, s);
-      k_pcg_update<X><<<vg, PCG_TPB, 0, s>>>(n, x, r, z, p, q, dinv, st, part, counter, tol, max_iter);
-      k_pcg_p<X><<<vg, PCG_TPB, 0, s>>>(n, p, z, st);
-      count_launch(2);
+      iterate<Op, double>(A, n, form, vg, x, W.r, W.zp, W.q, W.dinv, W.st, W.part, W.counter, tol, max_iter, s);
     }
     if (cudaError_t e = cudaGetLastError()) return (int)e;
     it_done += batch;
@@ -912,12 +1049,12 @@ static int pcg_persist(const NodeOp<double>& A, int64_t nnz, const double* b, do
   if (8 * nnz / G > lim || bitmap > lim) return 0;
   ulonglong2* slots = reinterpret_cast<ulonglong2*>(((uintptr_t)W.part + 15) & ~(uintptr_t)15);
   PersistArgs P{A.vbase, A.rowlen, A.dbase, A.mask, A.idx, A.val, A.n_nodes, n, x, W.r, W.q, W.dinv,
-                reinterpret_cast<ulonglong2*>(W.z), W.st, slots, reinterpret_cast<unsigned*>(slots + 2 * G),
+                reinterpret_cast<ulonglong2*>(W.zp), W.st, slots, reinterpret_cast<unsigned*>(slots + 2 * G),
                 reinterpret_cast<int64_t*>(slots + 2 * G + 1), tol,
                 max_iter, 0, 0};
-  spmv(A, (const double*)x, W.r, nullptr, nullptr, nullptr, 0, s);       // r = A x
-  k_pcg_setup<double><<<vec_grid<double>(n), PCG_TPB, 0, s>>>(n, b, W.r, W.z, nullptr, W.dinv, W.st, W.part, W.counter,
-                                                             W.q);
+  spmv(A, (const double*)x, W.r, s);                      // r = A x
+  k_pcg_setup<double><<<vec_grid<double>(n), PCG_TPB, 0, s>>>(n, b, W.r, W.zp, W.dinv, W.st, W.part, W.counter,
+                                                             FORM_TAGS, W.q);
   cudaMemsetAsync(slots, 0, sizeof(ulonglong2) * (2 * G + 1), s);
   cudaMemsetAsync(W.st + S_NEED, 0, sizeof(double), s);
   if (cudaError_t e = cudaFuncSetAttribute(k_persist_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitmap))
@@ -964,8 +1101,7 @@ static int pcg_fp64(const Op& A, int64_t n, const double* b, double* x, double t
   cudaMemsetAsync(W.counter, 0, 2 * sizeof(unsigned), s);
   diag_inv(A, W.dinv, jacobi, s);
   int it = 0;
-  int r = pcg_core<Op, double>(A, n, b, x, W.r, W.z, W.p, W.q, W.dinv, W.st, W.counter, W.part, tol, max_iter,
-                               check_every, &it, relres, s);
+  int r = pcg_core(A, n, b, x, W, tol, max_iter, check_every, &it, relres, s);
   if (iters) *iters = it;
   return r;
 }
@@ -990,15 +1126,16 @@ static int pcg_mixed(const Op64& A, const Op32& A32, int64_t n, const double* b,
   double* st2 = work + S_LEN + 2 + 5 * n + part_len(n);
   unsigned* counter2 = (unsigned*)(st2 + S_LEN);
   float* f = (float*)(st2 + S_LEN + 2);
-  float *xf = f, *rf = f + n, *zf = f + 2 * n, *pf = f + 3 * n, *qf = f + 4 * n;
+  float *xf = f, *rf = f + n, *qf = f + 4 * n;
+  float2* zpf = reinterpret_cast<float2*>(f + 2 * n);
   cudaMemsetAsync(W.counter, 0, 2 * sizeof(unsigned), s);
   cudaMemsetAsync(counter2, 0, 2 * sizeof(unsigned), s);
   diag_inv(A, W.dinv, 1, s);
   const unsigned vg = vec_grid<double>(n);
   const unsigned vgf = vec_grid<float>(n);
   // FP64 residual of the initial guess and the reference norm b.D^-1 b
-  spmv(A, (const double*)x, W.r, nullptr, nullptr, nullptr, 0, s);
-  k_pcg_setup<double><<<vg, PCG_TPB, 0, s>>>(n, b, W.r, W.z, W.p, W.dinv, W.st, W.part, W.counter);
+  spmv(A, (const double*)x, W.r, s);
+  k_pcg_setup<double><<<vg, PCG_TPB, 0, s>>>(n, b, W.r, W.zp, W.dinv, W.st, W.part, W.counter, FORM_ARRAYS, nullptr);
   count_launch();
   double h64[S_LEN];
   cudaMemcpyAsync(h64, W.st, sizeof(h64), cudaMemcpyDeviceToHost, s);
@@ -1012,7 +1149,8 @@ static int pcg_mixed(const Op64& A, const Op32& A32, int64_t n, const double* b,
     // FP32 start from r64: x32 = 0, r32 = r64, z32, p32, rho; stop test scale from b
     cudaMemsetAsync(xf, 0, sizeof(float) * n, s);
     cudaMemsetAsync(rf, 0, sizeof(float) * n, s);
-    k_pcg_setup<float><<<vgf, PCG_TPB, 0, s>>>(n, W.r, rf, zf, pf, W.dinv, st2, W.part, counter2);
+    const int form = form_for<float>(n);
+    k_pcg_setup<float><<<vgf, PCG_TPB, 0, s>>>(n, W.r, rf, zpf, W.dinv, st2, W.part, counter2, form, nullptr);
     count_launch();
     cudaMemcpyAsync(st2 + S_RZ0, W.st + S_RZ0, sizeof(double), cudaMemcpyDeviceToDevice, s);
     const int ce = std::max(1, check_every);
@@ -1020,14 +1158,7 @@ static int pcg_mixed(const Op64& A, const Op32& A32, int64_t n, const double* b,
     while (total < max_iter) {
       const int batch = std::min(ce, max_iter - total);
       for (int k = 0; k < batch; ++k) {
-        spmv(A32, (const float*)pf, qf, st2, W.part, counter2, 1, s);
-        k_pcg_update<float><<<vgf, PCG_TPB, 0, s>>>(n, xf, rf, zf, pf, qf, W.dinv, st2, W.part, counter2, 0.0,
-                                                   max_iter);
-        count_launch();
-        if (k + 1 < batch) {
-          k_pcg_p<float><<<vgf, PCG_TPB, 0, s>>>(n, pf, zf, st2);
-          count_launch();
-        }
+        iterate<Op32, float>(A32, n, form, vgf, xf, rf, zpf, qf, W.dinv, st2, W.part, counter2, 0.0, max_iter, s);
       }
       total += batch;
       if (inner_tol > 0.0 && total < max_iter) {
@@ -1036,19 +1167,15 @@ static int pcg_mixed(const Op64& A, const Op32& A32, int64_t n, const double* b,
         if (cudaError_t e = cudaStreamSynchronize(s)) return (int)e;
         const double rz32 = h32[S_RZ];
         if (h32[S_STATUS] != (double)FEA_EBREAKDOWN && rz32 > inner_tol * rz_last &&
-            rz32 / h64[S_RZ0] >= tol) {
-          k_pcg_p<float><<<vgf, PCG_TPB, 0, s>>>(n, pf, zf, st2);
-          count_launch();
+            rz32 / h64[S_RZ0] >= tol)
           continue;
-        }
       }
       // replacement: x64 += x32, r64 = b - A x64, r32 / z32 / rho / beta from it
       k_axpy_f32<<<grid_for(n, 256), 256, 0, s>>>(n, x, xf);
       cudaMemsetAsync(xf, 0, sizeof(float) * n, s);
-      spmv(A, (const double*)x, W.r, nullptr, nullptr, nullptr, 0, s);
-      k_mixed_replace<<<vg, PCG_TPB, 0, s>>>(n, b, W.r, W.dinv, rf, zf, W.st, st2, W.part, W.counter, tol);
-      k_pcg_p<float><<<vgf, PCG_TPB, 0, s>>>(n, pf, zf, st2);
-      count_launch(3);
+      spmv(A, (const double*)x, W.r, s);
+      k_mixed_replace<<<vg, PCG_TPB, 0, s>>>(n, b, W.r, W.dinv, rf, zpf, form, W.st, st2, W.part, W.counter, tol);
+      count_launch(2);
       ++nrep;
       double h32[S_LEN];
       cudaMemcpyAsync(h64, W.st, sizeof(h64), cudaMemcpyDeviceToHost, s);
@@ -1566,7 +1693,7 @@ extern "C" int fea_spmv(int64_t n, const int64_t* ip, const int32_t* ix, const d
   if (n == 0) return FEA_OK;
   int64_t nnz = 0;
   if (int r = read_nnz(ip, n, &nnz, s)) return r;
-  spmv(CsrOp<double>{ip, ix, v, n, nnz}, x, y, nullptr, nullptr, nullptr, 0, s);
+  spmv(CsrOp<double>{ip, ix, v, n, nnz}, x, y, s);
   return (int)cudaGetLastError();
 }
 
@@ -1574,7 +1701,7 @@ extern "C" int fea_spmv_nodes(const fea_nodes_t* N, const int32_t* ix, const dou
                               cudaStream_t s) {
   if (!nodes_ok(N) || !ix || !v || !x || !y) return FEA_EINVAL;
   if (N->ndof == 0) return FEA_OK;
-  spmv(node_op<double>(N, ix, v), x, y, nullptr, nullptr, nullptr, 0, s);
+  spmv(node_op<double>(N, ix, v), x, y, s);
   return (int)cudaGetLastError();
 }
 
@@ -1610,17 +1737,15 @@ extern "C" int fea_pcg_solve_nodes(const fea_nodes_t* N, const int32_t* ix, cons
   if (relres) *relres = 0.0;
   if (n == 0) return FEA_OK;
   const NodeOp<double> A = node_op<double>(N, ix, v);
-  if (((uintptr_t)work & 15) == 0) {             // (the pairs of k_pcg_persist are 16-byte aligned)
-    const PcgWork W = carve(work, n);
-    cudaMemsetAsync(W.counter, 0, 2 * sizeof(unsigned), s);
-    diag_inv(A, W.dinv, 1, s);
-    bool fits = false;
-    int it = 0;
-    const int r = pcg_persist(A, N->nnz, b, x, tol, max_iter, check_every, W, &fits, &it, relres, s);
-    if (iters) *iters = it;
-    if (fits || r != 0) return r;
-  }
-  return pcg_fp64(A, n, b, x, tol, max_iter, check_every, 1, work, iters, relres, s);
+  const PcgWork W = carve(work, n);
+  cudaMemsetAsync(W.counter, 0, 2 * sizeof(unsigned), s);
+  diag_inv(A, W.dinv, 1, s);
+  bool fits = false;
+  int it = 0;
+  int r = pcg_persist(A, N->nnz, b, x, tol, max_iter, check_every, W, &fits, &it, relres, s);
+  if (!fits && r == 0) r = pcg_core(A, n, b, x, W, tol, max_iter, check_every, &it, relres, s);
+  if (iters) *iters = it;
+  return r;
 }
 
 extern "C" int fea_pcg_solve_mixed(int64_t n, const int64_t* ip, const int32_t* ix, const double* v,

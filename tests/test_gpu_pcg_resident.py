@@ -98,8 +98,8 @@ def test_caps_guesses_and_breakdown():
 
 @pytest.mark.parametrize("shift", [0, 1])
 def test_work_buffer_bounds_and_alignment(shift):
-    """The buffer's tail is untouched; a work pointer that is not 16-byte
-    aligned takes the kernels per part, with the same solution."""
+    """The buffer's tail is untouched, also where the work pointer is not
+    16-byte aligned."""
     from fea_b200 import _lib as L
     P, K, b = system("C3D4", (7, 6, 5), "roller", True)
     wl = int(L.fea_pcg_work_len(P.ndof))
