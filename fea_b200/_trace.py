@@ -10,11 +10,15 @@ import os
 ENABLED = os.environ.get("FEA_B200_NVTX", "0") not in ("", "0")
 
 
-@contextlib.contextmanager
+_OFF = contextlib.nullcontext()
+
+
 def nvtx(name: str):
-    if not ENABLED:
-        yield
-        return
+    return _range(name) if ENABLED else _OFF
+
+
+@contextlib.contextmanager
+def _range(name: str):
     import torch
     torch.cuda.nvtx.range_push(name)
     try:

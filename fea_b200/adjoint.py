@@ -23,7 +23,7 @@ def _full(asm, reduced):
     """Reduced DOF vector -> all-DOF vector [N_total, 3] with zeros on
     Dirichlet and unused DOFs."""
     full = torch.zeros(asm.RGC_list_indexStart[-1], dtype=torch.float64, device=asm.device)
-    full[asm._remain_dev] = reduced
+    full[asm._remain_idx] = reduced
     return full.view(-1, 3)
 
 
@@ -38,7 +38,7 @@ def residual_vjp(asm, GC, lam):
     dmu = []
     for gi, e in enumerate(asm._mat_elems):
         mu, kappa = e.materials.parameters()
-        out = torch.zeros(1, dtype=torch.float64, device=asm.device)
+        out = torch.empty(1, dtype=torch.float64, device=asm.device)
         P.adjoint_vjp_volume(gi, mu, kappa, gc, lam_full, dX, out)
         dmu.append(out[0])
     for fi, ld in enumerate(asm._face_loads):
@@ -51,6 +51,8 @@ def _to_part_frames(asm, dX):
     instance evaluates its elements at X R^T (and its loads at X R^T + t), so
     the gradient with respect to X is the assembly-frame one times R."""
     for name, ins in asm._instances.items():
+        if not bool(ins._rotation.any()):
+            continue
         R = ins.rotation_matrix.to(torch.float64)
         if torch.equal(R, torch.eye(3, dtype=torch.float64)):
             continue
@@ -90,7 +92,7 @@ def compliance_gradient(asm, GC, pcg_tol=1e-26, pcg_max_iter=200000, return_lamb
     C = torch.dot(f, gc)
     u_full = _full(asm, gc)
     Hu = pressure_hvp(asm, gc, u_full)
-    rhs = (f - Hu.reshape(-1)[asm._remain_dev]).contiguous()
+    rhs = (f - Hu.reshape(-1)[asm._remain_idx]).contiguous()
     lam = torch.zeros_like(rhs)
     it, rr, st = P.pcg(K, rhs, lam, pcg_tol, pcg_max_iter, check_every=50)
     dX, dmu = residual_vjp(asm, gc, lam)

@@ -231,6 +231,8 @@ class Assembly:
         self.RGC_remain_index_flatten = torch.from_numpy(
             np.concatenate([r.reshape(-1) for r in self.RGC_remain_index]))
         self._remain_dev = self.RGC_remain_index_flatten.to(self.device)
+        # the same as positions: indexing with the mask would wait for its count
+        self._remain_idx = torch.nonzero(self.RGC_remain_index_flatten).flatten().to(self.device)
         self.GC = self._RGC2GC(self.RGC)
         self._GC_list_indexStart = np.cumsum([0] + [int(r.sum()) for r in self.RGC_remain_index]).tolist()
         self._build_plan()
@@ -265,7 +267,6 @@ class Assembly:
         plan_mask = np.concatenate(masks)
         self._plan = DevicePlan(torch.cat(X), plan_mask, groups, faces, device=self.device)
         self._Xinst = torch.cat(Xi).to(self.device).contiguous()
-        self._energy_buf = torch.zeros(1, dtype=torch.float64, device=self.device)
         self._system = None
         if self._constraints:
             tied = []
@@ -304,7 +305,7 @@ class Assembly:
     # -- GC <-> RGC (assembly.py:470-499) ---------------------------------------
     def _GC2RGC(self, GC):
         full = torch.zeros(self.RGC_list_indexStart[-1], dtype=torch.float64, device=self.device)
-        full[self._remain_dev] = GC.to(self.device, torch.float64)
+        full[self._remain_idx] = GC.to(self.device, torch.float64)
         RGC = [full[self.RGC_list_indexStart[i]:self.RGC_list_indexStart[i + 1]].view(self._RGC_size[i])
                for i in range(len(self._RGC_size))]
         for c in self._constraints.values():      # tied nodes follow their points (couple.py:34-40)
@@ -320,6 +321,8 @@ class Assembly:
             if RGC is None:
                 raise ValueError("Either RGC or GC must be provided.")
             GC = self._RGC2GC(RGC)
+        if isinstance(GC, torch.Tensor) and GC.dtype is torch.float64 and GC.device == self.device and GC.is_contiguous():
+            return GC
         return torch.as_tensor(GC, dtype=torch.float64).to(self.device).contiguous()
 
     # -- assembly ------------------------------------------------------------------
@@ -380,8 +383,9 @@ class Assembly:
         """sum of element energies + p V of every pressure load (assembly.py:389-415)."""
         P = self.plan
         gc = self._gc(RGC, GC)
-        total = torch.zeros((), dtype=torch.float64, device=self.device)
+        total = None
         if self._system is not None:
+            total = torch.zeros((), dtype=torch.float64, device=self.device)
             S = self._system
             gcr = gc
             gc = S.plan_gc(gcr)
@@ -391,14 +395,18 @@ class Assembly:
                     q = torch.zeros(6, dtype=torch.float64, device=self.device)
                     q[torch.as_tensor(keep, device=self.device)] = gcr[b0:b0 + keep.shape[0]]
                     total = total - (f[name] * q).sum()
+        # one value per group and load, each added in one launch
+        parts = torch.empty(len(self._mat_elems) + len(self._face_loads), dtype=torch.float64, device=self.device)
+        parts = parts.unbind()
         for gi, e in enumerate(self._mat_elems):
             mu, kappa = e.materials.parameters()
-            P.energy_volume(gi, mu, kappa, gc, self._energy_buf)
-            total = total + self._energy_buf[0]
+            P.energy_volume(gi, mu, kappa, gc, parts[gi])
+            total = parts[gi] if total is None else total + parts[gi]
         for fi, ld in enumerate(self._face_loads):
-            P.pressure_volume(fi, self._Xinst, gc, self._energy_buf)
-            total = total + float(ld.pressure) * self._energy_buf[0]
-        return total
+            v, p = parts[len(self._mat_elems) + fi], float(ld.pressure)
+            P.pressure_volume(fi, self._Xinst, gc, v)
+            total = p * v if total is None else torch.add(total, v, alpha=p)
+        return total if total is not None else torch.zeros((), dtype=torch.float64, device=self.device)
 
     # -- dynamics (assembly.py:187-206, 421-443) -----------------------------------
     def initialize_dynamic(self):

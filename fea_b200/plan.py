@@ -25,11 +25,12 @@ _NO_LOCK = contextlib.nullcontext()
 
 
 def vptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Handle of the calling thread's current stream on the current device."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def need(t, n, device, what):
@@ -39,6 +40,9 @@ def need(t, n, device, what):
     if t is None:
         return
     idx = device.index if device.index is not None else torch.cuda.current_device()
+    if (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype is torch.float64 and t.numel() >= n
+            and t.get_device() == idx and t.is_contiguous()):
+        return
     if (not isinstance(t, torch.Tensor) or t.dtype != torch.float64 or t.device.type != device.type
             or t.device.index != idx or not t.is_contiguous() or t.numel() < n):
         raise ValueError("%s: expected a contiguous float64 tensor of at least %d entries on %s, got %s" %
@@ -216,7 +220,7 @@ class DevicePlan:
             self._slots_len = max([g.slot_len for g in self.groups], default=0)
             self._slots = (torch.empty(self._slots_len, dtype=torch.float64, device=self.device)
                            if self._slots_len else None)
-            self._slots_stream = torch.cuda.current_stream().cuda_stream
+            self._slots_stream = stream()
             self._slots_lock = threading.Lock()
         self._scratch = None
         self._coo = None
@@ -258,8 +262,7 @@ class DevicePlan:
         host threads do not interleave, and the stream orders them); calls on
         other streams, or under capture, take a buffer of their own from the
         caching allocator."""
-        if n <= self._slots_len and not torch.cuda.is_current_stream_capturing() \
-                and torch.cuda.current_stream().cuda_stream == self._slots_stream:
+        if n <= self._slots_len and stream() == self._slots_stream and not torch.cuda.is_current_stream_capturing():
             return self._slots, n, self._slots_lock
         try:
             return torch.empty(n, dtype=torch.float64, device=self.device), n, _NO_LOCK
