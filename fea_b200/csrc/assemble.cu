@@ -1293,6 +1293,146 @@ __global__ void __launch_bounds__(128) k_face_rk(FaceParams P) {
   write_back<true>(P.chunkptr, P.chunklist, P.chunkdim, P.vbase, P.dbase, P.mask, P.soff, P.roff, ch, sm, P.K, nv, P.R);
 }
 
+// The same with 4 lanes per (row node, face): lane g evaluates Gauss point g
+// (frame, inverse, determinant, to shared memory), then lane b forms block b
+// and adds it to K itself, only the entries of the face's nodes, in rounds of
+// one incidence per node so that every entry is summed in incidence order.
+// The kernel above, a thread per incidence, adds through whole rows in shared
+// memory (9 times the entries of a solid's face) and serves the chunks of a
+// node with more than 32 faces.  Bound by latency (six dependent loads, then a
+// read-modify-write per round): one wave of CTAs up to some 20,000 faces (16
+// lanes per incidence: 24.0 us at 4,096 Q4 faces, two waves).  Against the
+// kernel above: 10.5 and 16.9 us at 4,096 Q4 faces, 7.4 and 17.1 at 480 T3
+// faces, 6.3 and 23 at 42 Q4 faces of shuffled nodes, 4.8 and 7.1 for R alone at
+// 2,304 Q4 faces.
+constexpr int FC_INC = 32;                       // incidences per chunk and CTA
+// Face<NF>::sf(g, m, a) by arithmetic: lanes of different g and a would take
+// turns at constant memory
+template <int NF>
+__device__ __forceinline__ double face_shape(int g, int m, int a) {
+  if (NF == 3) {
+    const double x = g == 1 ? 2.0 / 3.0 : 1.0 / 6.0, y = g == 2 ? 2.0 / 3.0 : 1.0 / 6.0;
+    if (m == 0) return a == 0 ? 1.0 - x - y : (a == 1 ? x : y);
+    return a == 0 ? -1.0 : (a == m ? 1.0 : 0.0);
+  }
+  const double q = 0.57735026918962576451;       // 1/sqrt(3)
+  const double xa = (a == 1 || a == 2) ? 1.0 : -1.0, ya = a >= 2 ? 1.0 : -1.0;
+  const double fx = 1.0 + xa * ((g == 1 || g == 2) ? q : -q), fy = 1.0 + ya * (g >= 2 ? q : -q);
+  return 0.25 * (m == 2 ? ya : fy) * (m == 1 ? xa : fx);
+}
+template <int NF>
+__global__ void __launch_bounds__(4 * FC_INC) k_face_rk4(FaceParams P) {
+  constexpr int NG = Face<NF>::NG;
+  __shared__ double tab[NG * 3 * NF];
+  __shared__ double gp[FC_INC][NG][10];
+  __shared__ double rs[FC_INC][3];
+  const int slot = threadIdx.x >> 2, l = threadIdx.x & 3;
+  const int i0 = P.chunkinc[blockIdx.x], i1 = P.chunkinc[blockIdx.x + 1];
+  const int q = i0 + slot;
+  const bool act = q < i1;
+  for (int t = threadIdx.x; t < NG * 3 * NF; t += 4 * FC_INC) tab[t] = face_shape<NF>(t / (3 * NF), t / NF % 3, t % NF);
+  __syncthreads();
+  int32_t cn[NF];
+  int a = 0, n = 0, rank = -1, L = 0;
+  unsigned mn = 0, mc = 0;
+  double* row = nullptr;
+  if (act) {
+    const int ea = P.inc[q];
+    const int64_t f = ea >> 4;
+    a = ea & 15;
+#pragma unroll
+    for (int c = 0; c < NF; ++c) cn[c] = P.conn[f * NF + c];
+    n = P.conn[f * NF + a];
+    rank = q - P.nodeinc[n];
+    mn = P.mask[n];
+    if (P.K && l < NF) {
+      const unsigned bo = P.boff[(int64_t)q * NF + l];
+      if (bo != 0xFFFFu) {
+        mc = P.mask[P.conn[f * NF + l]];
+        L = P.rowlen[n];
+        row = P.K + P.vbase[n] + bo;
+        for (int r = 0; r < popc3(mn); ++r) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (int64_t)r * L));
+      }
+    }
+    if (l < NG) {
+      double x[NF][3], r[9], inv[9];
+      face_nodes<NF>(P, cn, x);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) r[k] = 0.0;
+#pragma unroll
+      for (int c = 0; c < NF; ++c)
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          const double s = tab[(l * 3 + m) * NF + c];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) r[3 * k + m] += s * x[c][k];
+        }
+      const double det = inv3(r, inv);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) gp[slot][l][k] = inv[k];
+      gp[slot][l][9] = det;
+    }
+  }
+  __syncwarp();
+  double kacc[9], racc[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < 9; ++k) kacc[k] = 0.0;
+  if (act && l < NF) {
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      const double w3 = Face<NF>::w(g) / 3.0 * P.p;
+      const double* v = gp[slot][g];
+      const double det = v[9];
+      double B[3] = {0.0, 0.0, 0.0}, C[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        const double sa = tab[(g * 3 + m) * NF + a], sb = tab[(g * 3 + m) * NF + l];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          B[j] += sa * v[3 * m + j];
+          C[j] += sb * v[3 * m + j];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const double Ai = det * B[i], Di = det * C[i];
+        racc[i] += w3 * Ai;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) kacc[3 * i + j] += w3 * (Ai * C[j] - Di * B[j]);
+      }
+    }
+  }
+  if (P.R) {
+    if (act && l == 0) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) rs[slot][i] = racc[i];
+    }
+    __syncthreads();
+    if (rank == 0 && l < 3 && (mn >> l & 1u)) {    // the node's incidences are consecutive slots
+      double s = 0.0;
+      for (int t = slot; t < slot + P.nodeinc[n + 1] - q; ++t) s += rs[t][l];
+      P.R[P.dbase[n] + rank3(mn, l)] += s;
+    }
+  }
+  if (!P.K) return;
+  for (int k = 0; k < P.maxval; ++k) {
+    if (rank == k && row) {
+      double v[9];                                 // all loads, then the stores
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          v[3 * i + j] = (mn >> i & mc >> j & 1u) ? row[rank3(mn, i) * L + rank3(mc, j)] : 0.0;
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (mn >> i & mc >> j & 1u) row[rank3(mn, i) * L + rank3(mc, j)] = v[3 * i + j] + kacc[3 * i + j];
+    }
+    __syncthreads();
+  }
+}
+
 template <int NF>
 __global__ void __launch_bounds__(256) k_face_volume(FaceParams P, double* partial) {
   __shared__ double sh[256];
@@ -1904,6 +2044,14 @@ extern "C" int fea_assemble_pressure(const fea_nodes_t* N, const fea_group_t* G,
   FaceParams P = face_params(N, G, p, Xi, gc);
   P.K = K;
   P.R = R;
+  if (G->threads == FC_INC) {
+    if ((size_t)G->smem_doubles * sizeof(double) > (size_t)smem_limit()) return FEA_ESMEM;
+    if (G->nchunk <= 0) return FEA_OK;
+    if (G->kind == FEA_T3) k_face_rk4<3><<<(unsigned)G->nchunk, 4 * FC_INC, 0, st>>>(P);
+    else k_face_rk4<4><<<(unsigned)G->nchunk, 4 * FC_INC, 0, st>>>(P);
+    count_launch();
+    return (int)cudaGetLastError();
+  }
   if (G->kind == FEA_T3) return launch_chunked(k_face_rk<3>, G->nchunk, G->threads, G->smem_doubles, st, P);
   return launch_chunked(k_face_rk<4>, G->nchunk, G->threads, G->smem_doubles, st, P);
 }
