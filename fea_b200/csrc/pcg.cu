@@ -1233,7 +1233,8 @@ struct PcgbSlotDev {
   double* x;
   double* st;
   unsigned* counter;       // [0] SpMV items, [1] update items, [2] start chunks
-  double *dinv, *r, *z, *p, *q;
+  double *dinv, *r, *q;
+  double2* zp;             // (z, p_old) of every row
   double *part_s, *part_u, *part_0;
   const int64_t* vbase;    // plan layout (node rows), or NULL: plain CSR rows
   const int32_t* rowlen;
@@ -1316,6 +1317,10 @@ __device__ __forceinline__ double pcgb_warp_sum(const double* part, int n, int s
 // sums do not depend on the run it is processed in.  (With the register
 // count capped for 4 CTAs per SM the kernel ran 24% slower.)
 __device__ __forceinline__ void pcgb_nodes_spmv_run(const PcgbSlotDev& S, int g0, int cnt, int lane) {
+  PairVec<double> pv;
+  pv.zp = S.zp;
+  pv.st = S.st;
+  pv.init();
   const int h = lane >> 4, hl = lane & 15;
   const int64_t nbeg = (int64_t)g0 * PCGB_GROUP;
   const int64_t nend = min((int64_t)(g0 + cnt) * PCGB_GROUP, S.n_nodes);
@@ -1368,7 +1373,7 @@ __device__ __forceinline__ void pcgb_nodes_spmv_run(const PcgbSlotDev& S, int g0
         }
       double xv[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) xv[k] = hv[k] ? S.p[j[k]] : 0.0;
+      for (int k = 0; k < 3; ++k) xv[k] = hv[k] ? pv(j[k]) : 0.0;
       s0 += va[0][0] * xv[0] + va[0][1] * xv[1] + va[0][2] * xv[2];
       s1 += va[1][0] * xv[0] + va[1][1] * xv[1] + va[1][2] * xv[2];
       s2 += va[2][0] * xv[0] + va[2][1] * xv[1] + va[2][2] * xv[2];
@@ -1386,7 +1391,7 @@ __device__ __forceinline__ void pcgb_nodes_spmv_run(const PcgbSlotDev& S, int g0
       const int64_t r = S.dbase[nd] + hl;
       const double sr = hl == 0 ? s0 : (hl == 1 ? s1 : s2);
       S.q[r] = sr;
-      contrib += sr * S.p[r];
+      contrib += sr * pv(r);
     }
     nd = nx;
     m = m2;
@@ -1408,19 +1413,23 @@ template <int LANES>
 __device__ __forceinline__ double pcgb_rows_spmv(const PcgbSlotDev& S, int64_t r0, int64_t r1, int lane) {
   constexpr int RPP = 32 / LANES;
   const int sl = lane % LANES, sub = lane / LANES;
+  PairVec<double> pv;
+  pv.zp = S.zp;
+  pv.st = S.st;
+  pv.init();
   double contrib = 0.0;
   for (int64_t base = r0; base < r1; base += RPP) {
     const int64_t row = base + sub;
     double s = 0.0;
     if (row < r1) {
       const int64_t b = S.ptr[row], e = S.ptr[row + 1];
-      for (int64_t i = b + sl; i < e; i += LANES) s += S.val[i] * S.p[S.idx[i]];
+      for (int64_t i = b + sl; i < e; i += LANES) s += S.val[i] * pv(S.idx[i]);
     }
 #pragma unroll
     for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LANES);
     if (row < r1 && sl == 0) {
       S.q[row] = s;
-      contrib += s * S.p[row];
+      contrib += s * pv(row);
     }
   }
 #pragma unroll
@@ -1433,6 +1442,8 @@ __device__ __forceinline__ double pcgb_rows_spmv(const PcgbSlotDev& S, int64_t r
 // SpMV streams through a run's items without stopping at their boundaries,
 // and the slot's completion counter advances once per run.
 __global__ void __launch_bounds__(PCG_TPB) k_pcgb_spmv(PcgbView V) {
+  grid_next();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * PCG_WARPS;
   const int64_t nit = V.hdr->nitem_s;
@@ -1473,10 +1484,11 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcgb_spmv(PcgbView V) {
   }
 }
 
-// The vector kernels take contiguous runs of the update item list as the
-// SpMV does: the slot's pointers and scalars are read once per run and its
+// The update takes contiguous runs of the update item list as the SpMV does: the slot's pointers and scalars are read once per run and its
 // completion counter advances once per run.
 __global__ void __launch_bounds__(PCG_TPB) k_pcgb_update(PcgbView V) {
+  grid_next();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * PCG_WARPS;
   const int64_t nit = V.hdr->nitem_u;
@@ -1492,8 +1504,10 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcgb_update(PcgbView V) {
     const double alpha = S.st[S_ALPHA];
     double* __restrict__ x = S.x;
     double* __restrict__ r = S.r;
-    double* __restrict__ z = S.z;
-    const double* __restrict__ p = S.p;
+    double2* __restrict__ zp = S.zp;
+    PairVec<double> pf;
+    pf.st = S.st;
+    pf.init();
     const double* __restrict__ q = S.q;
     const double* __restrict__ dinv = S.dinv;
     const int64_t n = S.n;
@@ -1506,7 +1520,7 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcgb_update(PcgbView V) {
         const int64_t i = i0 + 32 * k;
         const bool in = i < n;
         xv[k] = in ? x[i] : 0.0;
-        pv[k] = in ? p[i] : 0.0;
+        pv[k] = in ? pf.of(zp[i]) : 0.0;         // the p that the SpMV multiplied
         rv[k] = in ? r[i] : 0.0;
         qv[k] = in ? q[i] : 0.0;
         dv[k] = in ? dinv[i] : 0.0;
@@ -1520,7 +1534,7 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcgb_update(PcgbView V) {
           const double ri = rv[k] - alpha * qv[k];
           r[i] = ri;
           const double zi = ri * dv[k];
-          z[i] = zi;
+          zp[i] = make_double2(zi, pv[k]);
           c += ri * zi;
         }
       }
@@ -1545,42 +1559,6 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcgb_update(PcgbView V) {
           S.st[S_DONE] = 1.0;
         }
         S.counter[1] = 0u;
-      }
-    }
-  }
-}
-
-__global__ void __launch_bounds__(PCG_TPB) k_pcgb_p(PcgbView V) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nw = (int64_t)gridDim.x * PCG_WARPS;
-  const int64_t nit = V.hdr->nitem_u;
-  const int64_t per = (nit + nw - 1) / nw;
-  int64_t it = ((int64_t)blockIdx.x * PCG_WARPS + (threadIdx.x >> 5)) * per;
-  const int64_t it_end = min(nit, it + per);
-  while (it < it_end) {                           // warp-uniform
-    const PcgbSlotDev& S = V.slots[V.u_slot[it]];
-    const int l0 = V.u_local[it];
-    const int cnt = (int)min(it_end - it, (int64_t)S.nitem_u - l0);
-    it += cnt;
-    if (S.st[S_DONE] != 0.0) continue;
-    const double beta = S.st[S_BETA];
-    double* __restrict__ p = S.p;
-    const double* __restrict__ z = S.z;
-    const int64_t n = S.n;
-    for (int l = l0; l < l0 + cnt; ++l) {
-      constexpr int K = PCGB_ROWS / 32;
-      double zv[K], pv[K];
-      const int64_t i0 = (int64_t)l * PCGB_ROWS + lane;
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const int64_t i = i0 + 32 * k;
-        zv[k] = i < n ? z[i] : 0.0;
-        pv[k] = i < n ? p[i] : 0.0;
-      }
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const int64_t i = i0 + 32 * k;
-        if (i < n) p[i] = zv[k] + beta * pv[k];
       }
     }
   }
@@ -1634,8 +1612,7 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcgb_start(PcgbView V, int32_t slot
     const double ri = S.b[i] - S.r[i];
     S.r[i] = ri;
     const double zi = ri * di;
-    S.z[i] = zi;
-    S.p[i] = zi;
+    S.zp[i] = make_double2(zi, 0.0);             // (beta = 0: p = z)
     c_rz = ri * zi;
     c_bb = S.b[i] * S.b[i] * di;
   }
@@ -1658,6 +1635,7 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcgb_start(PcgbView V, int32_t slot
       S.st[S_RZ0] = bb == 0.0 ? 1.0 : bb;
       S.st[S_ITER] = 0.0;
       S.st[S_STATUS] = 0.0;
+      S.st[S_BETA] = 0.0;
       S.st[S_DONE] = (bb == 0.0 || rz == 0.0 || rz / (bb == 0.0 ? 1.0 : bb) < S.tol || S.max_iter <= 0) ? 1.0 : 0.0;
       S.counter[2] = 0u;
     }
@@ -1845,7 +1823,11 @@ extern "C" int fea_pcgb_set(void* table, int32_t max_slots, int64_t max_items, i
     d.st = w;
     d.counter = (unsigned*)(w + S_LEN);
     d.dinv = w + S_LEN + 2;
-    d.r = d.dinv + h.n; d.z = d.r + h.n; d.p = d.z + h.n; d.q = d.p + h.n;
+    d.r = d.dinv + h.n;
+    double* zp = d.r + h.n;
+    zp += (uintptr_t)zp >> 3 & 1;                    // (16-byte pairs; the buffer ends with two spare doubles)
+    d.zp = reinterpret_cast<double2*>(zp);
+    d.q = zp + 2 * h.n;
     d.part_s = d.q + h.n; d.part_u = d.part_s + is; d.part_0 = d.part_u + iu;
     if (h.vbase_dev) { d.vbase = h.vbase_dev; d.rowlen = h.rowlen_dev; d.dbase = h.dbase_dev; d.mask = h.mask_dev; }
     d.n = h.n;
@@ -1906,12 +1888,10 @@ extern "C" int fea_pcgb_iterate(void* table, int32_t max_slots, int64_t max_item
   const int64_t warps_needed = max_items;
   const unsigned g1 = occ_grid(k_pcgb_spmv, warps_needed, PCG_WARPS);
   const unsigned g2 = occ_grid(k_pcgb_update, warps_needed, PCG_WARPS);
-  const unsigned g3 = occ_grid(k_pcgb_p, warps_needed, PCG_WARPS);
   for (int32_t k = 0; k < iters; ++k) {
-    k_pcgb_spmv<<<g1, PCG_TPB, 0, s>>>(V);
-    k_pcgb_update<<<g2, PCG_TPB, 0, s>>>(V);
-    k_pcgb_p<<<g3, PCG_TPB, 0, s>>>(V);
-    count_launch(3);
+    launch_after(k_pcgb_spmv, g1, PCG_TPB, s, V);
+    launch_after(k_pcgb_update, g2, PCG_TPB, s, V);
+    count_launch(2);
   }
   return (int)cudaGetLastError();
 }
