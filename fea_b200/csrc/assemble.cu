@@ -542,36 +542,43 @@ __global__ void __launch_bounds__(VolTPB<NN>::v) k_vol_rk(VolParams P) {
 }
 
 // ---- C3D8 R + K: element kernel + staged-block gather -----------------------
-// k_hex_elem evaluates every element ONCE: 8 lanes per element, lane g
-// computes the kinematics of Gauss point g and the vectors q_b = F^-T g_b,
-// f_b = F g_b of all 8 nodes into shared memory; then lane a builds the
-// upper-triangular blocks K_ab it owns (circulant assignment: b = a + d mod 8,
-// d = 0..3, plus d = 4 for a < 4 — 36 blocks over 8 lanes) with its own row
-// vectors in registers,
+// k_hex_elem evaluates every element once.  A warp takes four elements: 8
+// lanes per element evaluate its Gauss points (kinematics, the vectors q and f
+// of the 8 nodes and five scalars, to shared memory), then the whole
+// warp builds one element's tangent after the other with FP64 tensor
+// instructions.  With q_a = F^-T g_a, f_a = F g_a,
 //   K_ab = sum_g (A_a q_b^T + B_a f_b^T + q_b C_a^T + wc (g_a . g_b) I),
 //   A_a = w(alpha f_a + beta q_a), B_a = w alpha q_a, C_a = w gamma q_a,
-// and the element residual R_a = sum_g w(mu J^-2/3 f_a + c2 q_a).  Each lane
-// then writes its blocks from registers to their staged positions (the
-// plan's STAGEPOS), oriented to the upper node block (row node numbered
-// lower), and R_a to the incidence's slot of a separate array.  A node's
-// staged region lists, block-major, the contributions to each of its upper
-// blocks in element order; k_hex_gat copies the region to shared memory with
-// coalesced 16-byte copies, sums each upper block's contiguous contributions
-// and writes the block into the node's rows and its transpose into the
-// column node's rows: every CSR value written once.
-// g_b itself is not staged: g_a . g_b = (F^-1 f_a) . (F^T q_b) = f_a . q_b,
-// so a (Gauss point, node) slot holds 6 doubles and an element 456: 29,184
-// bytes of shared memory per CTA.  Six CTAs per SM: the launch bound holds
-// the kernel to 168 registers (64 threads x 6 CTAs x 168 <= 64K), 12 warps
-// per SM (k_hex_elem 544.3 -> 474.6 us at 64^3 against 45,568 bytes and five
-// CTAs).
-constexpr int HX_CTAS = 6;                // resident CTAs per SM the launch bound asks for
-constexpr int HX_EPB = 8;                 // elements per CTA
-constexpr int HX_TPB = 8 * HX_EPB;        // threads per CTA
-constexpr int HX_VB = 6;                  // doubles per (gp, node) vector slot: q, f (16-byte aligned)
-constexpr int HX_VG = 50;                 // doubles per Gauss point (8 slots + 2 pad: conflict-free rows)
-constexpr int HX_SC = 8 * HX_VG;          // offset of the per-Gauss-point scalars (6 each)
-constexpr int HX_EL = HX_SC + 48;         // doubles per element (6 scalars per Gauss point)
+// the 8 x 8 matrix of component (j, k) over the node pairs is a product over
+// the Gauss points, sum_g A_aj q_bk + B_aj f_bk + C_ak q_bj, plus on j = k the
+// matrix sum_gi wc f_ai q_bi (g_a . g_b = f_a . q_b).  In m8n8k4 a lane holds
+// node lane / 4 at Gauss point lane % 4 in both operands: it reads q and f of
+// that node at two Gauss points and holds every operand, no shared memory
+// between the products.  The six components j <= k suffice (K_ab[k, j] =
+// K_ba[j, k]): 36 instructions of 256 multiply-adds.  R_a = sum_g wc f_a + wc2 q_a.
+// The blocks go to shared memory, oriented to the upper node block (row node
+// numbered lower), and from there to their staged positions (the plan's
+// STAGEPOS), 27 and more lanes on consecutive values; R_a to the incidence's
+// slot of a separate array.  A node's staged region lists, block-major, the
+// contributions to each of its upper blocks in element order; k_hex_gat copies
+// the region to shared memory with coalesced 16-byte copies, sums each upper
+// block's contiguous contributions and writes the block into the node's rows
+// and its transpose into the column node's rows: every CSR value written once.
+// Bound by the FP64 pipe and the latency of the chains of products at 16 warps
+// an SM: the tensor instructions run at the rate of the FP64 units (64
+// multiply-adds a cycle and SM) but need a fifth of the issue slots and no
+// shared memory for operands (FP64 pipes 58 %, shared-memory wavefronts 46 % of
+// peak).  64^3 elements: 348 us, 397 us with the same products in FP64
+// registers; 362.8 us with the blocks at the plan's numbers in shared memory
+// (37 % of the store wavefronts bank conflicts), 368 us with the operands
+// formed from the maps in the second phase.
+constexpr int HX_CTAS = 4;                // resident CTAs per SM (128 registers, 53 KB; with 3: 399.5 against 362.8 us)
+constexpr int HX_WARPS = 4;               // warps per CTA, of up to four elements each
+constexpr int64_t HX_WAVE = 148 * HX_CTAS * HX_WARPS;   // warps the B200 holds at once
+constexpr int HX_TPB = 32 * HX_WARPS;     // threads per CTA
+constexpr int HX_SC = 8 * 8 * 6;          // doubles of the q and f of an element's 8 Gauss points and nodes, before
+constexpr int HX_EL = HX_SC + 40;         // its scalars, 5 x 8 Gauss points (8 mod 16: two elements' stores share no bank)
+constexpr size_t HX_SMEM = sizeof(double) * 4 * HX_WARPS * HX_EL;
 constexpr int HX_GW = 4;                  // warps per gather CTA
 // Gather lanes per row node: 16 (two nodes per warp: 397.0 against 461.4 us
 // with 32 lanes per node at 64^3, where rows hold 27 blocks and regions 36),
@@ -583,242 +590,229 @@ constexpr int HX_LPN = 16;
 __host__ __device__ inline int64_t hx_rslot_base(int64_t nblk) { return (nblk * 9 + 1) & ~(int64_t)1; }
 constexpr int HX_GINC = 32;               // chunk capacity of C3D8 plans (the C3D8 kernels read no chunks)
 
+// c += A B of 8x4 and 4x8 FP64 operands: a is A[lane / 4][lane % 4], b is
+// B[lane % 4][lane / 4], c holds C[lane / 4][2 (lane % 4) + 0, 1]
+__device__ __forceinline__ void mma_f64(double c[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+// double2 c (of 3: q0 q1, q2 f0, f1 f2) of node a at Gauss point g in the
+// element's area: the rotation by g puts the 8 lanes of a 16-byte access, 8
+// Gauss points (writing) or 2 nodes x 4 Gauss points (reading), on 8 banks
+__device__ __forceinline__ int hx_unit(int c, int g, int a) { return 64 * c + 8 * g + ((a + 2 * (g & 3) + (g >> 2)) & 7); }
+
+// Place of the block of local nodes a, b among the 36 of an element in shared
+// memory: no two blocks that a half warp stores together (a of 0..3 or 4..7, b
+// even or odd) are congruent mod 16, so its 9 odd-strided 8-byte stores touch
+// every bank at most once, however the nodes are numbered.
+__device__ alignas(2) const uint8_t HX_PLACE[64] = {
+    1, 2, 6, 15, 3, 10, 9, 22, 2, 0, 5, 19, 16, 7, 4, 25, 6, 5, 13, 11, 14, 17, 8, 12, 15, 19, 11, 20, 26, 24, 28, 30,
+    3, 16, 14, 26, 18, 31, 32, 27, 10, 7, 17, 24, 31, 35, 29, 34, 9, 4, 8, 28, 32, 29, 23, 21, 22, 25, 12, 30, 27, 34, 21, 33};
+// ... and the plan's number (owner_slot) of the block at each place
+__device__ const uint8_t HX_AT[36] = {5,  0,  1,  4,  31, 6,  2,  9, 14, 30, 27, 11, 35, 10, 12, 3,  8,  13,
+                                      20, 7,  15, 29, 33, 28, 17, 34, 16, 23, 18, 25, 19, 21, 22, 32, 26, 24};
+
 template <bool ER>
 __global__ void __launch_bounds__(HX_TPB, HX_CTAS) k_hex_elem(VolParams P, double* __restrict__ stage,
-                                                     double* __restrict__ rslot) {
-  __shared__ __align__(16) double sv[HX_EPB * HX_EL];
-  const double q3 = 0.57735026918962576451;   // 1/sqrt(3)
-  const int le = threadIdx.x >> 3;
-  const int lane = threadIdx.x & 7;
-  const int64_t e = (int64_t)blockIdx.x * HX_EPB + le;
-  const bool act = e < P.ne;
-  double* V = sv + le * HX_EL;
-  // ---- phase 0: node `lane`'s coordinates and displacement, once per element,
-  // to the scalar area of V (48 doubles: 6 per node) for all 8 lanes --------
+                                                             double* __restrict__ rslot, int epw) {
+  extern __shared__ __align__(16) double hxs[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t e0 = ((int64_t)blockIdx.x * HX_WARPS + warp) * epw;
+  const int n = (int)(P.ne - e0 < epw ? P.ne - e0 : epw);   // elements of this warp
   int32_t cl = 0;
-  if (act) {
-    cl = P.conn[e * 8 + lane];
-    const double* xb = P.X + 3 * (int64_t)cl;
-    const unsigned mb = P.mask[cl];
-    const int32_t rb = P.rdof[cl];
-    double2* o = reinterpret_cast<double2*>(V + HX_SC + lane * 6);
-    o[0] = make_double2(__ldg(xb), __ldg(xb + 1));
-    o[1] = make_double2(__ldg(xb + 2), node_u(P.gc, rb, mb, 0));
-    o[2] = make_double2(node_u(P.gc, rb, mb, 1), node_u(P.gc, rb, mb, 2));
-  }
-  __syncwarp();
-  // ---- phase 1: Gauss point g = lane ----------------------------------------
-  const double px = csx(lane) * q3, py = csy(lane) * q3, pz = csz(lane) * q3;
-  const double fxp = 1.0 + px, fxm = 1.0 - px, fyp = 1.0 + py, fym = 1.0 - py, fzp = 1.0 + pz, fzm = 1.0 - pz;
-  double J0[9], Ju[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) J0[i] = Ju[i] = 0.0;
-  // dN_b/dxi at this Gauss point, once for both node loops: 12 products of
-  // two shape factors (with the 1/8), signed per node (the same bits as
-  // 0.125 * s * f * f')
-  double dxs[8][3];
   {
-    const double yz[4] = {0.125 * fym * fzm, 0.125 * fyp * fzm, 0.125 * fym * fzp, 0.125 * fyp * fzp};
-    const double xz[4] = {0.125 * fxm * fzm, 0.125 * fxp * fzm, 0.125 * fxm * fzp, 0.125 * fxp * fzp};
-    const double xy[4] = {0.125 * fxm * fym, 0.125 * fxp * fym, 0.125 * fxm * fyp, 0.125 * fxp * fyp};
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const int ix = ((b + 1) >> 1) & 1, iy = (b >> 1) & 1, iz = b >> 2;
-      dxs[b][0] = ix ? yz[iy + 2 * iz] : -yz[iy + 2 * iz];
-      dxs[b][1] = iy ? xz[ix + 2 * iz] : -xz[ix + 2 * iz];
-      dxs[b][2] = iz ? xy[ix + 2 * iy] : -xy[ix + 2 * iy];
+    // ---- Gauss points: 8 lanes per element -----------------------------------
+    const int sub = lane >> 3, l8 = lane & 7;
+    const int64_t e = e0 + sub;
+    const bool act = sub < n;
+    double* V = hxs + (4 * warp + sub) * HX_EL;
+    if (act) {
+      cl = P.conn[e * 8 + l8];
+      const double* xb = P.X + 3 * (int64_t)cl;
+      const unsigned mb = P.mask[cl];
+      const int32_t rb = P.rdof[cl];
+      double2* o = reinterpret_cast<double2*>(V + 6 * l8);
+      o[0] = make_double2(__ldg(xb), __ldg(xb + 1));
+      o[1] = make_double2(__ldg(xb + 2), node_u(P.gc, rb, mb, 0));
+      o[2] = make_double2(node_u(P.gc, rb, mb, 1), node_u(P.gc, rb, mb, 2));
     }
-  }
-  if (act) {
+    __syncwarp();
+    const HexLane<double> H(l8);
+    double JJ[2][9];
+    if (act) hex_gradients<double, 2>(H, V, JJ);
+    __syncwarp();                                // the node data are read: the area takes q, f and the scalars
+    if (act) {
+      double iJ[9], F[9], iF[9], Jm;
+      const double w = inv3(JJ[0], iJ);          // Gauss weight 1
+      const double* Ju = JJ[1];
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const double d0 = dxs[b][0], d1 = dxs[b][1], d2 = dxs[b][2];
-      const double2* xs = reinterpret_cast<const double2*>(V + HX_SC + b * 6);
-      const double2 v0 = xs[0], v1 = xs[1], v2 = xs[2];
-      const double xv[3] = {v0.x, v0.y, v1.x}, uv[3] = {v1.y, v2.x, v2.y};
+      for (int I = 0; I < 3; ++I)
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const double x = xv[i], u = uv[i];
-        J0[3 * i] += x * d0; J0[3 * i + 1] += x * d1; J0[3 * i + 2] += x * d2;
-        Ju[3 * i] += u * d0; Ju[3 * i + 1] += u * d1; Ju[3 * i + 2] += u * d2;
-      }
-    }
-  }
-  __syncwarp();                                  // the node data are read: the area takes the scalars
-  if (act) {
-    double iJ[9], F[9], iF[9];
-    const double w = inv3(J0, iJ);             // Gauss weight 1
+        for (int i = 0; i < 3; ++i)
+          F[3 * I + i] = fma(Ju[3 * I], iJ[i], fma(Ju[3 * I + 1], iJ[3 + i], fma(Ju[3 * I + 2], iJ[6 + i], I == i ? 1.0 : 0.0)));
+      const double J = inv3_jm(F, iF, &Jm);      // F^-1 and J^-2/3 from one reciprocal cube root
+      const double mu = P.mu, kappa = P.kappa;
+      double sF2 = 0.0;
 #pragma unroll
-    for (int I = 0; I < 3; ++I)
+      for (int i = 0; i < 9; ++i) sF2 += F[i] * F[i];
+      const double I1 = Jm * sF2, muJm = mu * Jm;
+      double* S = V + HX_SC + l8;
+      S[0] = w * (-2.0 / 3.0 * muJm);                                   // w alpha
+      S[8] = w * (kappa * J * (2.0 * J - 1.0) + 2.0 / 9.0 * mu * I1);    // w beta
+      S[16] = w * (mu * I1 / 3.0 - kappa * J * (J - 1.0));                // w gamma
+      S[24] = w * muJm;                                                   // w c (delta term, residual)
+      S[32] = w * (kappa * J * (J - 1.0) - mu * I1 / 3.0);                // w c2 (residual)
+      // Mq = J0^-1 F^-1, Mf = J0^-1 F^T: q_b = Mq^T dxi_b, f_b = Mf^T dxi_b
+      double Mq[9], Mf[9];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        F[3 * I + i] = fma(Ju[3 * I], iJ[i], fma(Ju[3 * I + 1], iJ[3 + i], fma(Ju[3 * I + 2], iJ[6 + i], I == i ? 1.0 : 0.0)));
-    double Jm;
-    const double J = inv3_jm(F, iF, &Jm);      // F^-1 and J^-2/3 from one reciprocal cube root
-    const double mu = P.mu, kappa = P.kappa;
-    double sF2 = 0.0;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) sF2 += F[i] * F[i];
-    const double I1 = Jm * sF2, muJm = mu * Jm;
-    double* S = V + HX_SC + lane * 6;
-    S[0] = w * (-2.0 / 3.0 * muJm);                                 // w alpha
-    S[1] = w * (kappa * J * (2.0 * J - 1.0) + 2.0 / 9.0 * mu * I1);  // w beta
-    S[2] = w * (mu * I1 / 3.0 - kappa * J * (J - 1.0));              // w gamma
-    S[3] = w * muJm;                                                 // w c (delta term, residual)
-    S[4] = w * (kappa * J * (J - 1.0) - mu * I1 / 3.0);              // w c2 (residual)
-    S[5] = (double)cl;                                               // node `lane`, for phase 3
-    // Mq = J0^-1 F^-1, Mf = J0^-1 F^T: q_b = Mq^T dxi_b, f_b = Mf^T dxi_b, g_b = J0^-T dxi_b
-    double Mq[9], Mf[9];
-#pragma unroll
-    for (int m = 0; m < 3; ++m)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        Mq[3 * m + k] = iJ[3 * m] * iF[k] + iJ[3 * m + 1] * iF[3 + k] + iJ[3 * m + 2] * iF[6 + k];
-        Mf[3 * m + k] = iJ[3 * m] * F[3 * k] + iJ[3 * m + 1] * F[3 * k + 1] + iJ[3 * m + 2] * F[3 * k + 2];
-      }
-    double* Vg = V + lane * HX_VG;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const double d0 = dxs[b][0], d1 = dxs[b][1], d2 = dxs[b][2];
-      double v[6];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        v[k] = d0 * Mq[k] + d1 * Mq[3 + k] + d2 * Mq[6 + k];
-        v[3 + k] = d0 * Mf[k] + d1 * Mf[3 + k] + d2 * Mf[6 + k];
-      }
-      double2* o = reinterpret_cast<double2*>(Vg + b * HX_VB);   // 16-byte aligned slot
-      o[0] = make_double2(v[0], v[1]);
-      o[1] = make_double2(v[2], v[3]);
-      o[2] = make_double2(v[4], v[5]);
-    }
-  }
-  __syncwarp();
-  // ---- phase 2: row node a = lane (lanes of an inactive element idle) --------
-  const int a = lane;
-  const int nb = a < 4 ? 5 : 4;
-  int32_t spos[5] = {-1, -1, -1, -1, -1};      // staged positions of the lane's blocks, loaded early
-  int32_t ipos = -1;
-  if (act) {
-    const int32_t* sp = P.stagepos + e * 36 + (a < 4 ? 5 * a : 20 + 4 * (a - 4));
-#pragma unroll
-    for (int d = 0; d < 5; ++d)
-      if (d < nb) spos[d] = sp[d];
-    ipos = P.incpos[e * 8 + a];
-  }
-  double acc[5][9];
-  double racc[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-  for (int d = 0; d < 5; ++d)
-#pragma unroll
-    for (int i = 0; i < 9; ++i) acc[d][i] = 0.0;
-#pragma unroll 1
-  for (int g = 0; g < (act ? 8 : 0); ++g) {
-    const double2* S2 = reinterpret_cast<const double2*>(V + HX_SC + g * 6);   // 16-byte aligned
-    const double2 s01 = S2[0], s23 = S2[1], s45 = S2[2];
-    const double wa = s01.x, wb = s01.y, wg = s23.x, wc = s23.y, wc2 = s45.x;
-    const double* Va = V + g * HX_VG + a * HX_VB;
-    double qa[3], fa[3], gm[3], A[3], B[3], Cc[3];
-    {
-      const double2* v2 = reinterpret_cast<const double2*>(Va);
-      const double2 x0 = v2[0], x1 = v2[1], x2 = v2[2];
-      qa[0] = x0.x; qa[1] = x0.y; qa[2] = x1.x; fa[0] = x1.y; fa[1] = x2.x; fa[2] = x2.y;
-      gm[0] = wc * fa[0]; gm[1] = wc * fa[1]; gm[2] = wc * fa[2];       // w mu J^-2/3 f_a
-    }
-    double AC[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      A[k] = wa * fa[k] + wb * qa[k];
-      B[k] = wa * qa[k];
-      Cc[k] = wg * qa[k];
-      AC[k] = A[k] + Cc[k];
-      racc[k] = fma(wc, fa[k], racc[k]);
-      racc[k] = fma(wc2, qa[k], racc[k]);
-    }
-#pragma unroll
-    for (int d = 0; d < 5; ++d) {
-      const double* Vb = V + g * HX_VG + ((a + d) & 7) * HX_VB;
-      double qb[3], fb[3];
-      {
-        const double2* v2 = reinterpret_cast<const double2*>(Vb);
-        const double2 x0 = v2[0], x1 = v2[1], x2 = v2[2];
-        qb[0] = x0.x; qb[1] = x0.y; qb[2] = x1.x; fb[0] = x1.y; fb[1] = x2.x; fb[2] = x2.y;
-      }
-      const double dg = gm[0] * qb[0] + gm[1] * qb[1] + gm[2] * qb[2];    // w mu J^-2/3 g_a . g_b
-      // three fused multiply-adds into each accumulator, the delta term on
-      // the diagonal alone: 33 FP64 operations per block and Gauss point.
-      // d = 0 (K_aa = wa (f q^T + q f^T) + (wb + wg) q q^T + dg I, symmetric)
-      // takes the upper triangle with two FMAs an entry (18), d = 4 the upper
-      // triangle (24): at d = 4 every lane computes one, lane a < 4 that of K_a,a+4 and
-      // lane a + 4 that of K_a+4,a, whose strict part is the strict lower
-      // triangle of K_a,a+4 transposed (the two lanes share the block)
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
+      for (int m = 0; m < 3; ++m)
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          if ((d == 0 || d == 4) && k < j) continue;
-          double t = acc[d][3 * j + k];
-          if (d == 0) {                          // K_aa: fa_j B_k + qa_j (A_k + C_k), two FMAs
-            t = fma(fa[j], B[k], t);
-            t = fma(qa[j], AC[k], t);
-          } else {
-            t = fma(A[j], qb[k], t);
-            t = fma(B[j], fb[k], t);
-            t = fma(qb[j], Cc[k], t);
-          }
-          acc[d][3 * j + k] = t;
+          Mq[3 * m + k] = iJ[3 * m] * iF[k] + iJ[3 * m + 1] * iF[3 + k] + iJ[3 * m + 2] * iF[6 + k];
+          Mf[3 * m + k] = iJ[3 * m] * F[3 * k] + iJ[3 * m + 1] * F[3 * k + 1] + iJ[3 * m + 2] * F[3 * k + 2];
         }
-      acc[d][0] += dg;
-      acc[d][4] += dg;
-      acc[d][8] += dg;
-    }
-  }
-  // the strict lower triangle of K_a,a+4 from lane a + 4 (all lanes shuffle)
-  const int partner = (lane + 4) & 7;
-  const double l10 = __shfl_sync(0xffffffffu, acc[4][1], partner, 8);
-  const double l20 = __shfl_sync(0xffffffffu, acc[4][2], partner, 8);
-  const double l21 = __shfl_sync(0xffffffffu, acc[4][5], partner, 8);
-  acc[0][3] = acc[0][1];
-  acc[0][6] = acc[0][2];
-  acc[0][7] = acc[0][5];
-  acc[4][3] = l10;
-  acc[4][6] = l20;
-  acc[4][7] = l21;
-  // ---- phase 3: every block from registers to its staged position ------------
-  // K_ab as computed when the column node is numbered above the row node (or
-  // b = a), transposed when below, K_ab + K_ab^T when the element repeats
-  // the node (a != b); R_a to the incidence's residual slot.
-  if (act) {
-    const double na = V[HX_SC + a * 6 + 5];
+      double2* o = reinterpret_cast<double2*>(V);
 #pragma unroll
-    for (int d = 0; d < 5; ++d) {
-      if (d == 4 && nb == 4) break;
-      if (spos[d] < 0) continue;
-      const double nc = V[HX_SC + ((a + d) & 7) * 6 + 5];
-      double* out = stage + (int64_t)spos[d] * 9;
-      if (d == 0 || nc > na) {
+      for (int b = 0; b < 8; ++b) {
+        const double d0 = H.dxi(b, 0), d1 = H.dxi(b, 1), d2 = H.dxi(b, 2);
+        double v[6];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) out[i] = acc[d][i];
-      } else if (nc < na) {
+        for (int k = 0; k < 3; ++k) {
+          v[k] = d0 * Mq[k] + d1 * Mq[3 + k] + d2 * Mq[6 + k];
+          v[3 + k] = d0 * Mf[k] + d1 * Mf[3 + k] + d2 * Mf[6 + k];
+        }
 #pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-          for (int k = 0; k < 3; ++k) out[3 * j + k] = acc[d][3 * k + j];
-      } else {
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-          for (int k = 0; k < 3; ++k) out[3 * j + k] = acc[d][3 * j + k] + acc[d][3 * k + j];
+        for (int c = 0; c < 3; ++c) o[hx_unit(c, l8, b)] = make_double2(v[2 * c], v[2 * c + 1]);
       }
     }
-    if (ipos >= 0) {
-      double2* ro = reinterpret_cast<double2*>(rslot + (int64_t)ipos * 4);
-      ro[0] = make_double2(racc[0], racc[1]);
-      ro[1] = make_double2(racc[2], 0.0);
-    }
+    __syncwarp();
   }
-  if (ER && act) {
+  // ---- tangent of one element after the other: the whole warp ------------------
+  const int a = lane >> 2, g0 = lane & 3;         // this lane's node and Gauss points g0, g0 + 4
+  const int b0 = 2 * g0;                          // its columns of the products: nodes b0, b0 + 1
+  const uchar2 place = *reinterpret_cast<const uchar2*>(HX_PLACE + 2 * lane);
+  const int at0 = HX_AT[lane], at1 = HX_AT[32 + (lane & 3)];
+  int32_t p0 = 0, p1 = 0, ipos = 0;               // the next element's positions, one element ahead
+  if (n > 0) {
+    p0 = P.stagepos[e0 * 36 + at0];
+    p1 = P.stagepos[e0 * 36 + at1];
+    ipos = P.incpos[e0 * 8 + a];
+  }
+#pragma unroll 1
+  for (int sub = 0; sub < n; ++sub) {
+    const int64_t e = e0 + sub;
+    double* B = hxs + (4 * warp + sub) * HX_EL;   // the element's area: later its blocks
+    int32_t* ps = reinterpret_cast<int32_t*>(B + HX_SC);   // and their staged positions
+    double q[2][3], f[2][3], sc[2][5];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) P.elemR[(int64_t)(3 * a + j) * P.ne + e] = racc[j];
+    for (int h = 0; h < 2; ++h) {
+      const int g = g0 + 4 * h;
+      const double2* v = reinterpret_cast<const double2*>(B);
+      const double2 v0 = v[hx_unit(0, g, a)], v1 = v[hx_unit(1, g, a)], v2 = v[hx_unit(2, g, a)];
+      q[h][0] = v0.x; q[h][1] = v0.y; q[h][2] = v1.x;
+      f[h][0] = v1.y; f[h][1] = v2.x; f[h][2] = v2.y;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) sc[h][k] = B[HX_SC + 8 * k + g];
+    }
+    double r[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      r[k] = sc[0][3] * f[0][k] + sc[0][4] * q[0][k] + sc[1][3] * f[1][k] + sc[1][4] * q[1][k];
+    // sum_gi wc f_ai q_bi, where the three diagonal components start
+    double c[6][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) mma_f64(c[0], sc[h][3] * f[h][k], q[h][k]);
+    c[3][0] = c[5][0] = c[0][0];
+    c[3][1] = c[5][1] = c[0][1];
+    // components (j, k) = 00 01 02 11 12 22
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      double A[3], Bq[3], C[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        A[k] = sc[h][0] * f[h][k] + sc[h][1] * q[h][k];
+        Bq[k] = sc[h][0] * q[h][k];
+        C[k] = sc[h][2] * q[h][k];
+      }
+#pragma unroll
+      for (int j = 0, t = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = j; k < 3; ++k, ++t) {
+          mma_f64(c[t], k == j ? A[j] + C[j] : A[j], q[h][k]);
+          mma_f64(c[t], Bq[j], f[h][k]);
+          if (k != j) mma_f64(c[t], C[k], q[h][j]);
+        }
+    }
+    // ---- blocks to shared memory: K_ab's six from the lane of (a, b) when a's node
+    // is numbered below b's, the other three from the lane of (b, a); K_ab +
+    // K_ab^T when the element repeats the node (a != b) -----------------------------
+    const int32_t na = __shfl_sync(0xffffffffu, cl, 8 * sub + a);
+    bool twice = false;
+    __syncwarp();                                 // (q, f and the scalars are read)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int b = b0 + k;
+      const int32_t nb = __shfl_sync(0xffffffffu, cl, 8 * sub + b);
+      double* o = B + 9 * (k ? place.y : place.x);
+      if (na < nb || a == b || (na == nb && a < b)) {
+        o[0] = c[0][k];
+        o[1] = c[1][k];
+        o[2] = c[2][k];
+        o[4] = c[3][k];
+        o[5] = c[4][k];
+        o[8] = c[5][k];
+      }
+      if (na > nb || a == b || (na == nb && a < b)) {
+        o[3] = c[1][k];
+        o[6] = c[2][k];
+        o[7] = c[4][k];
+      }
+      twice |= na == nb && a != b;
+    }
+    ps[lane] = p0;
+    if (lane < 4) ps[32 + lane] = p1;
+    const int32_t slot = ipos;
+    if (sub + 1 < n) {
+      p0 = P.stagepos[(e + 1) * 36 + at0];
+      p1 = P.stagepos[(e + 1) * 36 + at1];
+      ipos = P.incpos[(e + 1) * 8 + a];
+    }
+    __syncwarp();
+    if (__any_sync(0xffffffffu, twice)) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int b = b0 + k;
+        const int32_t nb = __shfl_sync(0xffffffffu, cl, 8 * sub + b);
+        if (na == nb && a > b) {
+          double* o = B + 9 * (k ? place.y : place.x);
+          const double up[9] = {c[0][k], c[1][k], c[2][k], c[1][k], c[3][k], c[4][k], c[2][k], c[4][k], c[5][k]};
+#pragma unroll
+          for (int i = 0; i < 9; ++i) o[i] += up[i];
+        }
+      }
+      __syncwarp();
+    }
+    // ---- and to their staged positions -------------------------------------------
+#pragma unroll
+    for (int t0 = 0; t0 < 324; t0 += 32) {
+      const int t = t0 + lane;
+      if (t < 324) {
+        const int s = (t * 57) >> 9;              // t / 9
+        const int32_t at = ps[s];
+        if (at >= 0) stage[(int64_t)at * 9 + (t - 9 * s)] = B[t];
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) r[k] += __shfl_xor_sync(0xffffffffu, r[k], o);
+    if (slot >= 0 && g0 < 2)
+      reinterpret_cast<double2*>(rslot + (int64_t)slot * 4)[g0] = g0 ? make_double2(r[2], 0.0) : make_double2(r[0], r[1]);
+    if (ER && g0 < 3) P.elemR[(int64_t)(3 * a + g0) * P.ne + e] = g0 == 0 ? r[0] : (g0 == 1 ? r[1] : r[2]);
   }
 }
 
@@ -1933,10 +1927,17 @@ extern "C" int fea_assemble_volume(const fea_nodes_t* N, const fea_group_t* G, d
       const size_t gbytes = (size_t)HX_GW * (32 / lpn) * region;
       if (gbytes > (size_t)smem_limit()) return FEA_ESMEM;
       double* rslot = work + hx_rslot_base(G->nblk);
-      const unsigned grid = (unsigned)((G->ne + HX_EPB - 1) / HX_EPB);
+      // Elements per warp: below half a wave of warps one, so that an element's
+      // products do not wait for three others (210 elements: 4.3 against 7.5 us with
+      // four); with four the Gauss points use the whole warp (2,197 elements: 8.1, 6.6
+      // and 7.9 us with 1, 2 and 4; 4,096: 12.6, 10.7 and 9.4; 64^3: 641, 449 and 348).
+      const int epw = G->ne <= HX_WAVE / 2 ? 1 : G->ne <= HX_WAVE ? 2 : 4;
+      const unsigned grid = (unsigned)((G->ne + HX_WARPS * epw - 1) / (HX_WARPS * epw));
       if (grid) {
-        if (er) k_hex_elem<true><<<grid, HX_TPB, 0, st>>>(P, work, rslot);
-        else k_hex_elem<false><<<grid, HX_TPB, 0, st>>>(P, work, rslot);
+        auto ek = er ? k_hex_elem<true> : k_hex_elem<false>;
+        if (cudaError_t ce = cudaFuncSetAttribute(ek, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HX_SMEM))
+          return (int)ce;
+        ek<<<grid, HX_TPB, HX_SMEM, st>>>(P, work, rslot, epw);
         count_launch();
         if (cudaError_t ce = cudaGetLastError()) return (int)ce;
       }

@@ -178,3 +178,32 @@ def test_explicit_steps(dims, fp32):
     tol = 1e-4 if fp32 else TOL * 10
     for x, y in zip(*out):
         assert float((x - y).abs().max()) <= tol * float(x.abs().max())
+
+
+@pytest.mark.parametrize("dims", MESHES + [(13, 8, 11), (12, 11, 12), (14, 13, 13)])
+@pytest.mark.parametrize("repeat", [False, True])
+def test_tangent_and_residual(dims, repeat):
+    """One, two (1,185 elements and more) and four (2,369 and more) elements
+    per warp, with accumulate and the element residual."""
+    P, gc = hex_plan(dims, repeat=repeat)
+    g, N = P.groups[0], P.n_nodes
+    X, el = P.X.cpu().view(N, 3), g.conn.cpu().view(-1, 8).long()
+    m = O.Model(X, [O.Group("C3D8", el, 1.0, 40.0)], [], [])
+    m._free = (P.mask.cpu().view(N, 1) >> torch.arange(3) & 1).bool().reshape(-1)
+    used = torch.zeros(N, 3, dtype=torch.bool)    # a node of no element keeps what R held
+    used[el] = True
+    used = used.reshape(-1)[m.free_mask()]
+    R0, (ip, ix, K0) = m.assemble(gc.cpu())
+    assert torch.equal(P.indices.cpu().long(), ix.long())
+    e0 = O.element_residual_tangent("C3D8", X, el, m.gc_to_u(gc.cpu()), 1.0, 40.0, False)[0]
+    for acc in (False, True):
+        K, R = torch.full((P.nnz,), 0.5, dtype=torch.float64, device="cuda"), torch.full_like(gc, 0.25)
+        eR = torch.zeros(24 * g.ne, dtype=torch.float64, device="cuda")
+        P.assemble_volume(0, 1.0, 40.0, gc, K=K, R=R, elemR=eR, accumulate=acc)
+        assert float((K.cpu() - (0.5 if acc else 0.0) - K0).abs().max()) <= TOL * float(K0.abs().max())
+        d = (R.cpu() - (0.25 if acc else 0.0) - R0)[used]
+        assert float(d.abs().max()) <= TOL * max(1.0, float(R0.abs().max()))
+        assert close(eR.cpu(), e0.reshape(-1))
+        K2 = torch.full_like(K, 0.5)
+        P.assemble_volume(0, 1.0, 40.0, gc, K=K2, accumulate=acc)
+        assert torch.equal(K, K2)
