@@ -134,7 +134,7 @@ __device__ __forceinline__ void hex_store_slot(double* __restrict__ slot, int64_
 // node, one per component and one idle: with a thread per node the sum waited
 // on one load after the other at 15 warps per SM (48^3 block: 10.7 -> 7.3 us).
 constexpr int HL_SUM_TPB = 256;
-__device__ __forceinline__ double hex_sum_slots(const double* __restrict__ slot, const int32_t* __restrict__ inc,
+__device__ __forceinline__ double hex_sum_slots(const double* slot, const int32_t* __restrict__ inc,
                                                 int q0, int q1, int j) {
   constexpr int U = 8;
   double r = 0.0;

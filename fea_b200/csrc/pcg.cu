@@ -113,24 +113,6 @@ struct PairOf<double> { typedef double2 type; };
 template <>
 struct PairOf<float> { typedef float2 type; };
 
-// Programmatic dependent launch: a kernel's start overlaps the end of the one
-// before it; grid_wait() holds it until that one's results are there.
-__device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <class... P, class... Q>
-static void launch_after(void (*k)(P...), unsigned grid, unsigned threads, cudaStream_t s, Q... q) {
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3(threads);
-  c.stream = s;
-  cudaLaunchAttribute a[1];
-  a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  a[0].val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = a;
-  c.numAttrs = 1;
-  cudaLaunchKernelEx(&c, k, P(q)...);
-}
-
 // block sum: warp shuffles, then the 8 warp sums in fixed order
 __device__ __forceinline__ double block_sum_w(double v, double* sh) {
 #pragma unroll

@@ -511,11 +511,11 @@ int fea_ls_select(int64_t n, const double* E_dev, int32_t k0, double c1, double 
  * init == 0: on entry u = u_k, vh = vh_{k-1/2}, a = a_k.
  * Runs `steps` steps and leaves u, vh, a, v at the final step.
  * fp32 != 0 evaluates the element force in FP32 with FP64 nodal sums.
- * work_dev: fea_explicit_work_len(nodes) doubles, 16-byte aligned (a second
- * u buffer and two node-major copies of the coordinates and u, which the
- * element math reads with 16-byte loads).  With
- * fea_explicit_group_work_len(nodes, group) doubles a C3D8 group's elements
- * are evaluated once per step (else once per node).
+ * work_dev: fea_explicit_work_len(nodes) doubles, 16-byte aligned (two
+ * node-major copies of the coordinates and u, which the element math reads
+ * with 16-byte loads; the first ndof doubles are not used).  With
+ * fea_explicit_group_work_len(nodes, group) doubles the elements are
+ * evaluated once per step (else once per node).
  * ------------------------------------------------------------------------- */
 int64_t fea_explicit_work_len(const fea_nodes_t* nodes);
 int64_t fea_explicit_group_work_len(const fea_nodes_t* nodes, const fea_group_t* group);

@@ -111,3 +111,42 @@ def test_lists_of_the_host_plan():
     cl, tp = hp.array(L.G_BASE + L.A_CHUNKLIST), hp.array(L.FEA_A_G_TILEPTR)
     assert tp[0] == 0 and tp[-1] == len(cl) and np.all(np.diff(tp) > 0) and len(tp) > 3
     assert np.all(np.diff([nodeinc[n] for n in cl[tp[:-1]]] + [nodeinc[-1]]) <= 128)
+
+
+@gpu
+@pytest.mark.parametrize("kind", [(1, 1, 1), (2, 1, 1), (11, 1, 2), (9, 8, 7), "fan"])
+@pytest.mark.parametrize("fp32", [0, 1])
+def test_explicit_steps(kind, fp32):
+    """A start and five steps: the short work buffer (every node evaluates its
+    elements) and the long one (each element once; counts around the 32 of a
+    warp and the 128 of a block)."""
+    from fea_b200 import DevicePlan
+    from fea_b200 import _lib as L
+    X, el = mesh(kind)
+    N = len(X)
+    mask = np.full(N, 7, np.uint8)
+    mask[N // 2], mask[N // 3], mask[-1] = 0, 5, 2
+    P = DevicePlan(X, mask, [("C3D4", el)])
+    g = P.groups[0]
+    h = 1 if kind == "fan" else 1 / max(kind)
+    gc = torch.from_numpy(np.random.default_rng(2).normal(0, 5e-3 * h, P.ndof)).cuda()
+    v0 = 1e-2 * torch.randn(P.ndof, dtype=torch.float64, generator=torch.Generator().manual_seed(5)).cuda()
+    minv = P.lumped_mass_inv([1.0])
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    short = int(L.fea_explicit_work_len(C.byref(P.nodes)))
+    n = int(L.fea_explicit_group_work_len(C.byref(P.nodes), C.byref(g.desc)))
+    assert n == short + 9 * g.ne
+    out = []
+    for wn in (short, n):
+        pad = torch.full((wn + 64,), 7.25, dtype=torch.float64, device="cuda")
+        u, v, vh, a = gc.clone(), v0.clone(), torch.empty_like(gc), torch.empty_like(gc)
+        for init, steps in ((1, 2), (0, 3)):
+            L.check(L.fea_explicit_run(C.byref(P.nodes), C.byref(g.desc), 1.0, 30.0, ptr(minv), 2e-3 * h, steps, fp32,
+                                       init, ptr(u), ptr(vh), ptr(a), ptr(v), ptr(pad), wn, st), "explicit")
+        assert bool((pad[wn:] == 7.25).all())
+        out.append((u, v, a))
+    # FP64: the paths order the products of an element differently (1e-15 of its stresses' terms, which cancel by up
+    # to a factor of a hundred).  FP32: kappa * 6e-8 of the stresses' scale, which the strains' 1e-2 magnifies
+    tol = 2e-3 if fp32 else TOL * 10
+    for x, y in zip(*out):
+        assert float((x - y).abs().max()) <= tol * float(x.abs().max())
