@@ -1,13 +1,14 @@
 // Element residual / tangent assembly, follower pressure, energy and lumped
 // mass for C3D4 / C3D8 Neo-Hookean groups (sm_100a, FP64).
 //
-// Assembly is a per-node-row GATHER: every (row node n, incident element e)
-// pair ("incidence") gets one thread, which evaluates the element at all its
-// Gauss points and accumulates the 3 x (3 nn) strip K_e[a(n), :] in
-// registers.  The strips of one node are summed in shared memory in a fixed
-// order (incidence rank), and the chunk's rows — a contiguous range of the
-// reduced CSR values — are written to HBM exactly once.  No atomics, no
-// colouring, bitwise-deterministic results.
+// Assembly is a per-node-row GATHER.  C3D4: every (row node n, incident element
+// e) pair ("incidence") gets one thread, which evaluates the 3 x 12 strip
+// K_e[a(n), :]; a CTA sums the strips of its nodes per column block in a fixed
+// order from shared memory (k_tet_rk).  C3D8: every element is evaluated once
+// and its blocks (or nodal residuals) are staged per node, then summed per
+// node (k_hex_elem + k_hex_gat, k_hex_force + k_hex_force_sum).  Every CSR
+// value is written to HBM exactly once.  No atomics, no colouring,
+// bitwise-deterministic results.
 //
 // Reference behaviour reproduced (FEA = sssnnn7119/FEA):
 //   F, J, J^-2/3, I1          Element_3D.components_Solid   C3base.py:454-480

@@ -435,9 +435,7 @@ struct NodeOp32q {
 // LPN lanes per node (32 / LPN nodes per warp), 4 columns per lane per
 // pass: the next nodes' metadata are loaded while the current ones are
 // processed; loops and shuffles warp-uniform.
-#ifndef FEA_F32Q_LPN
-#define FEA_F32Q_LPN 8
-#endif
+constexpr int F32Q_LPN = 8;
 template <int LPN, class X, class Vec>
 __global__ void __launch_bounds__(PCG_TPB, 4) k_spmv_node32q(NodeOp32q A, Vec x, X* __restrict__ y,
                                                              double* st, double* part, unsigned* counter, int mode) {
@@ -878,7 +876,7 @@ static void spmv_on(const NodeOp<V>& A, Vec x, X* y, double* st, double* part, u
 template <class X, class Vec>
 static void spmv_on(const NodeOp32q& A, Vec x, X* y, double* st, double* part, unsigned* counter, int mode,
                     cudaStream_t s) {
-  constexpr int LPN = FEA_F32Q_LPN;
+  constexpr int LPN = F32Q_LPN;
   auto k = k_spmv_node32q<LPN, X, Vec>;
   launch_after(k, occ_grid(k, A.n_nodes, PCG_WARPS * (32 / LPN)), PCG_TPB, s, A, x, y, st, part, counter, mode);
   count_launch();
@@ -1008,14 +1006,12 @@ static int smem_optin() {
 
 // CTAs of k_pcg_persist: one per SM, fewer when a CTA would own less than
 // PP_ROWS rows (a smaller grid sums faster).
-#ifndef FEA_PP_ROWS
-#define FEA_PP_ROWS 72
-#endif
+constexpr int PP_ROWS = 72;
 static unsigned persist_grid(int64_t n) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::min(sms, PP_MAXG), n / FEA_PP_ROWS));
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::min(sms, PP_MAXG), n / PP_ROWS));
 }
 
 // PCG on a matrix that fits the shared memory of the grid's CTAs; *fits = false
@@ -1202,10 +1198,7 @@ static int read_nnz(const int64_t* ip, int64_t n, int64_t* nnz, cudaStream_t s) 
 // order with no block-level barrier.  A slot's arithmetic depends only on
 // its own items, so its iterates are the same bits alone or batched.
 constexpr int PCGB_ROWS = 256;      // rows per update item and per start chunk
-#ifndef FEA_PCGB_GROUP
-#define FEA_PCGB_GROUP 16
-#endif
-constexpr int PCGB_GROUP = FEA_PCGB_GROUP;   // nodes (plan layout) or rows (CSR) per SpMV item
+constexpr int PCGB_GROUP = 16;   // nodes (plan layout) or rows (CSR) per SpMV item
 
 struct PcgbSlotDev {
   const int64_t* ptr;

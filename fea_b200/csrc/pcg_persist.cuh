@@ -36,16 +36,10 @@
 // (included by pcg.cu after the S_* state indices)
 namespace fea {
 
-#ifndef FEA_PP_TPB
-#define FEA_PP_TPB 512
-#endif
-constexpr int PP_TPB = FEA_PP_TPB;
+constexpr int PP_TPB = 512;
 constexpr int PP_WARPS = PP_TPB / 32;
 constexpr int PP_MAXG = 256;              // CTAs, one per SM
-#ifndef FEA_PP_LPN
-#define FEA_PP_LPN 8
-#endif
-constexpr int PP_LPN = FEA_PP_LPN, PP_NPW = 32 / PP_LPN;   // lanes per node in the SpMV, nodes per warp
+constexpr int PP_LPN = 8, PP_NPW = 32 / PP_LPN;   // lanes per node in the SpMV, nodes per warp
 static_assert(PP_WARPS <= 16, "warp_sum<8>");
 constexpr int PP_SPIN = 1 << 22;          // polls, of about a microsecond each
 
