@@ -1328,7 +1328,7 @@ __global__ void __launch_bounds__(4 * FC_INC) k_face_rk4(FaceParams P) {
   for (int t = threadIdx.x; t < NG * 3 * NF; t += 4 * FC_INC) tab[t] = face_shape<NF>(t / (3 * NF), t / NF % 3, t % NF);
   __syncthreads();
   int32_t cn[NF];
-  int a = 0, n = 0, rank = -1, L = 0;
+  int a = 0, n = 0, rank = -1, L = 0, nb = -1 - l;   // nb: the column node of lane l
   unsigned mn = 0, mc = 0;
   double* row = nullptr;
   if (act) {
@@ -1341,9 +1341,10 @@ __global__ void __launch_bounds__(4 * FC_INC) k_face_rk4(FaceParams P) {
     rank = q - P.nodeinc[n];
     mn = P.mask[n];
     if (P.K && l < NF) {
+      nb = P.conn[f * NF + l];
       const unsigned bo = P.boff[(int64_t)q * NF + l];
       if (bo != 0xFFFFu) {
-        mc = P.mask[P.conn[f * NF + l]];
+        mc = P.mask[nb];
         L = P.rowlen[n];
         row = P.K + P.vbase[n] + bo;
         for (int r = 0; r < popc3(mn); ++r) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (int64_t)r * L));
@@ -1395,6 +1396,26 @@ __global__ void __launch_bounds__(4 * FC_INC) k_face_rk4(FaceParams P) {
 #pragma unroll
         for (int j = 0; j < 3; ++j) kacc[3 * i + j] += w3 * (Ai * C[j] - Di * B[j]);
       }
+    }
+  }
+  if (P.K) {
+    // A face that repeats a node (a collapsed Q4): the lanes of one node hold the
+    // same columns, and the lowest adds them all, in lane order.
+    int own = l;
+#pragma unroll
+    for (int t = 2; t >= 0; --t)
+      if (__shfl_sync(0xffffffffu, nb, t, 4) == nb) own = min(own, t);
+    if (__any_sync(0xffffffffu, own != l)) {
+#pragma unroll
+      for (int t = 1; t < 4; ++t) {
+        const int to = __shfl_sync(0xffffffffu, own, t, 4);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+          const double v = __shfl_sync(0xffffffffu, kacc[k], t, 4);
+          if (to == l && t != l) kacc[k] += v;
+        }
+      }
+      if (own != l) row = nullptr;
     }
   }
   if (P.R) {
