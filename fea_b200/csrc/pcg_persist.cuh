@@ -11,8 +11,8 @@
 // take 6.6k and the SpMV 2.7k (shared-memory reads and their conflicts).  Here every CTA
 // owns a contiguous range of nodes with about the same number of values and
 // keeps, for the whole launch, in shared memory: the values and (renumbered)
-// columns of its rows, its rows of x, r, q and 1/|d|, and p of every column
-// that its rows touch.  An iteration is
+// columns of its rows, its rows of x, r, q and 1/|d|, and p of its rows
+// and of every column that they touch.  An iteration is
 //   p = z + beta p of the touched columns (z of other CTAs' rows through L2)
 //   q = A p, p.q   | alpha
 //   x, r, z, r.z   | beta, stop test
@@ -206,9 +206,11 @@ __host__ __device__ inline PersistLayout persist_layout(int64_t n, int64_t nodes
   return y;
 }
 
-// Marks the columns of the CTA's nodes in a bitmap over all rows (bm: words,
-// zeroed here); returns how many there are, with their running count before
-// each word in pre (if not NULL).  The whole block; ends with a barrier.
+// Marks the columns of the CTA's nodes and its own rows (a free node of no
+// element has an empty row, and p and z of every own row are kept) in a bitmap
+// over all rows (bm: words, zeroed here); returns how many there are, with their
+// running count before each word in pre (if not NULL).  The whole block; ends
+// with a barrier.
 __device__ __forceinline__ int mark_columns(PersistShared& S, const PersistArgs& A, int64_t n0, int nn, unsigned* bm,
                                             int* pre) {
   const int tid = threadIdx.x;
@@ -224,6 +226,7 @@ __device__ __forceinline__ int mark_columns(PersistShared& S, const PersistArgs&
       atomicOr(bm + (c >> 5), 1u << (c & 31));
     }
   }
+  for (int r = A.dbase[n0] + tid; r < A.dbase[n0 + nn]; r += PP_TPB) atomicOr(bm + (r >> 5), 1u << (r & 31));
   __syncthreads();
   const int per = (W + PP_TPB - 1) / PP_TPB;
   int mine = 0, total = 0;
@@ -324,7 +327,7 @@ __global__ void __launch_bounds__(PP_TPB, 1) k_pcg_persist(PersistArgs A) {
       kc[d.coff + q] = (uint16_t)(pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u)));
     }
   }
-  // (a row's own column is among its columns: the CTA's rows are consecutive touched columns)
+  // (the CTA's rows are consecutive touched columns)
   const int own = rows ? pre[row0 >> 5] + __popc(bm[row0 >> 5] & ((1u << (row0 & 31)) - 1u)) : 0;
   __syncthreads();                               // the bitmap is read: the values take its place
   double* kv = reinterpret_cast<double*>(smraw + persist_layout(A.n, nact, rows, ncol, touched, nval).vals);

@@ -96,6 +96,49 @@ def test_caps_guesses_and_breakdown():
     assert P.pcg(K, bad, torch.zeros_like(b), 1e-20, 100, raise_on_breakdown=False)[2] == L.FEA_EBREAKDOWN
 
 
+@pytest.mark.parametrize("kind,dims,extra", [("C3D8", (1, 1, 1), 1), ("C3D4", (5, 4, 3), 40), ("C3D8", (12, 9, 8), 300)])
+def test_free_nodes_without_elements(kind, dims, extra):
+    """Free nodes that no element holds (empty rows, a zero right-hand side) at
+    the start, in the middle and at the end of the numbering, alone and in
+    runs: they stay at their start value 0 and the others' solution is that
+    of the mesh without them."""
+    from fea_b200 import DevicePlan
+    from fea_b200.meshes import hex_block, tet_block
+    P, K, b = system(kind, dims, "roller")
+    _, el = (hex_block if kind == "C3D8" else tet_block)(0, dims=dims)
+    X, mask = P.X.cpu().numpy(), P.mask.cpu().numpy()
+    N = len(X)
+    at = np.unique(np.concatenate([[0, N // 2, N], np.linspace(1, N - 1, 5).astype(int)]))    # runs before these nodes
+    new = np.zeros(N, np.int64)
+    shift = 0
+    keep = np.ones(N + extra * len(at), bool)
+    for n in range(N + 1):
+        if n in at:
+            keep[n + shift:n + shift + extra] = False
+            shift += extra
+        if n < N:
+            new[n] = n + shift
+    X2 = np.zeros((len(keep), 3))
+    m2 = np.where(np.arange(len(keep)) % 3 == 0, 2, 7).astype(np.uint8)     # (some of them free in y only)
+    X2[keep], m2[keep] = X, mask
+    Q = DevicePlan(X2, m2, [(kind, new[el])])
+    assert Q.nnz == P.nnz
+    f = ((m2[:, None] >> np.arange(3)) & 1).astype(bool)
+    rows = torch.from_numpy(np.nonzero(np.repeat(keep[:, None], 3, 1)[f])[0]).cuda()
+    b2 = Q.zeros(Q.ndof)
+    b2[rows] = b
+    x, xa, xb = torch.zeros_like(b), torch.zeros_like(b2), torch.zeros_like(b2)
+    it = P.pcg(K, b, x, 1e-20, 20000)
+    ia = Q.pcg(K, b2, xa, 1e-20, 20000)
+    ib = Q.pcg(K, b2, xb, 1e-20, 20000, generic=True)
+    assert it[2] == ia[2] == ib[2] == 0 and abs(ia[0] - ib[0]) <= 2 + ib[0] // 50
+    other = torch.ones_like(b2, dtype=torch.bool)
+    other[rows] = False
+    assert not xa[other].any() and not xb[other].any()
+    for y in (xa[rows], xb[rows]):
+        assert float((y - x).abs().max()) <= 1e-7 * float(x.abs().max())
+
+
 @pytest.mark.parametrize("shift", [0, 1])
 def test_work_buffer_bounds_and_alignment(shift):
     """The buffer's tail is untouched, also where the work pointer is not
