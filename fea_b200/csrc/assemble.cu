@@ -1867,23 +1867,9 @@ static int launch_chunked(void (*kern)(Prm), int64_t nchunk, int threads, int64_
                           const Prm& p) {
   size_t bytes = (size_t)smem_doubles * sizeof(double);
   if (bytes > (size_t)smem_limit()) return FEA_ESMEM;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (err != cudaSuccess) return (int)err;
+  if (cudaError_t err = allow_smem((const void*)kern)) return (int)err;
   if (nchunk <= 0) return 0;
   kern<<<(unsigned)nchunk, threads, bytes, st>>>(p);
-  count_launch();
-  return (int)cudaGetLastError();
-}
-
-template <class Prm, class X>
-static int launch_chunked_ex(void (*kern)(Prm, X), int64_t nchunk, int threads, int64_t smem_doubles,
-                             cudaStream_t st, const Prm& p, X extra) {
-  size_t bytes = (size_t)smem_doubles * sizeof(double);
-  if (bytes > (size_t)smem_limit()) return FEA_ESMEM;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (err != cudaSuccess) return (int)err;
-  if (nchunk <= 0) return 0;
-  kern<<<(unsigned)nchunk, threads, bytes, st>>>(p, extra);
   count_launch();
   return (int)cudaGetLastError();
 }
@@ -1957,8 +1943,7 @@ extern "C" int fea_assemble_volume(const fea_nodes_t* N, const fea_group_t* G, d
       const unsigned grid = (unsigned)((G->ne + HX_WARPS * epw - 1) / (HX_WARPS * epw));
       if (grid) {
         auto ek = er ? k_hex_elem<true> : k_hex_elem<false>;
-        if (cudaError_t ce = cudaFuncSetAttribute(ek, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HX_SMEM))
-          return (int)ce;
+        if (cudaError_t ce = allow_smem((const void*)ek)) return (int)ce;
         ek<<<grid, HX_TPB, HX_SMEM, st>>>(P, work, rslot, epw);
         count_launch();
         if (cudaError_t ce = cudaGetLastError()) return (int)ce;
@@ -1975,8 +1960,7 @@ extern "C" int fea_assemble_volume(const fea_nodes_t* N, const fea_group_t* G, d
                                : (acc ? k_hex_gat<false, true, HX_LPN, false> : k_hex_gat<false, false, HX_LPN, false>))
                          : (wr ? (acc ? k_hex_gat<true, true, 32, false> : k_hex_gat<true, false, 32, false>)
                                : (acc ? k_hex_gat<false, true, 32, false> : k_hex_gat<false, false, 32, false>)));
-        if (cudaError_t ce = cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gbytes))
-          return (int)ce;
+        if (cudaError_t ce = allow_smem((const void*)gk)) return (int)ce;
         gk<<<g2, HX_GW * 32, gbytes, st>>>(P, work, rslot, capb, capq);
         count_launch();
       }
@@ -1992,8 +1976,7 @@ extern "C" int fea_assemble_volume(const fea_nodes_t* N, const fea_group_t* G, d
                     : (er ? k_tet_rk<true, false, true> : k_tet_rk<true, false, false>))
              : (acc ? (er ? k_tet_rk<false, true, true> : k_tet_rk<false, true, false>)
                     : (er ? k_tet_rk<false, false, true> : k_tet_rk<false, false, false>));
-      if (cudaError_t ce = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TET_SMEM))
-        return (int)ce;
+      if (cudaError_t ce = allow_smem((const void*)k)) return (int)ce;
       k<<<(unsigned)G->ntile, TET_TPB, TET_SMEM, st>>>(
           P, TetLists{G->clist_dev, reinterpret_cast<const uint2*>(G->crec_dev), G->crecptr_dev, G->tileptr_dev});
       count_launch();

@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cmath>
 #include <mutex>
+#include <unordered_map>
 
 #include "../../include/fea_b200.h"
 
@@ -189,6 +190,31 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 }
 
 inline int grid_for(int64_t n, int bs) { return (int)((n + bs - 1) / bs); }
+
+// Lets kernel k take all the dynamic shared memory that a block of the current
+// device has beside k's static part (*most bytes); each launch passes what it
+// needs.  Set once per device and kernel: the attribute belongs to the function,
+// and with a value per call another host thread's smaller one could come between
+// this thread's setting and its launch.
+inline cudaError_t allow_smem(const void* k, int64_t* most = nullptr) {
+  static std::mutex mu;
+  static std::unordered_map<const void*, int> done[64];
+  int dev = 0, optin = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  auto& m = done[dev & 63];
+  auto it = m.find(k);
+  if (it == m.end()) {
+    cudaFuncAttributes a;
+    if (cudaError_t e = cudaFuncGetAttributes(&a, k)) return e;
+    if (cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) return e;
+    const int v = optin - (int)a.sharedSizeBytes;
+    if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, v)) return e;
+    it = m.emplace(k, v).first;
+  }
+  if (most) *most = it->second;
+  return cudaSuccess;
+}
 
 // Programmatic dependent launch: a kernel's start overlaps the end of the one
 // before it; grid_wait() holds it until that one's results are there.

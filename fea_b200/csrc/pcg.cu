@@ -997,13 +997,6 @@ static int pcg_core(const Op& A, int64_t n, const double* b, double* x, const Pc
   return (int)host[S_STATUS];
 }
 
-static int smem_optin() {
-  int dev = 0, v = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return v;
-}
-
 // CTAs of k_pcg_persist: one per SM, fewer when a CTA would own less than
 // PP_ROWS rows (a smaller grid sums faster).
 constexpr int PP_ROWS = 72;
@@ -1022,9 +1015,11 @@ static int pcg_persist(const NodeOp<double>& A, int64_t nnz, const double* b, do
   *fits = false;
   const int64_t n = A.n;
   const unsigned G = persist_grid(n);
-  const int64_t lim = smem_optin() - (int64_t)sizeof(PersistShared) - 64;
+  int64_t lim = 0, lim_plan = 0;
+  if (cudaError_t e = allow_smem((const void*)k_pcg_persist, &lim)) return (int)e;
+  if (cudaError_t e = allow_smem((const void*)k_persist_plan, &lim_plan)) return (int)e;
   const int64_t bitmap = 4 * ((n + 31) / 32);
-  if (8 * nnz / G > lim || bitmap > lim) return 0;
+  if (8 * nnz / G > lim || bitmap > lim_plan) return 0;
   ulonglong2* slots = reinterpret_cast<ulonglong2*>(((uintptr_t)W.part + 15) & ~(uintptr_t)15);
   PersistArgs P{A.vbase, A.rowlen, A.dbase, A.mask, A.idx, A.val, A.n_nodes, n, x, W.r, W.q, W.dinv,
                 reinterpret_cast<ulonglong2*>(W.zp), W.st, slots, reinterpret_cast<unsigned*>(slots + 2 * G),
@@ -1035,8 +1030,6 @@ static int pcg_persist(const NodeOp<double>& A, int64_t nnz, const double* b, do
                                                              FORM_TAGS, W.q);
   cudaMemsetAsync(slots, 0, sizeof(ulonglong2) * (2 * G + 1), s);
   cudaMemsetAsync(W.st + S_NEED, 0, sizeof(double), s);
-  if (cudaError_t e = cudaFuncSetAttribute(k_persist_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitmap))
-    return (int)e;
   k_persist_plan<<<G, PP_TPB, (size_t)bitmap, s>>>(P);
   count_launch(2);
   if (cudaError_t e = cudaGetLastError()) return (int)e;
@@ -1055,8 +1048,6 @@ static int pcg_persist(const NodeOp<double>& A, int64_t nnz, const double* b, do
       if (need > (unsigned long long)lim) return 0;
       *fits = true;
       P.smem = (unsigned)need;
-      if (cudaError_t e = cudaFuncSetAttribute(k_pcg_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need))
-        return (int)e;
     }
     if (host[S_FAIL] != 0.0) return FEA_ETIMEOUT;
     if (host[S_DONE] != 0.0 || it_done >= max_iter) break;

@@ -179,3 +179,42 @@ def test_solves_on_two_streams():
     [t.start() for t in th]
     [t.join() for t in th]
     assert torch.equal(out[0], ref[0]) and torch.equal(out[1], ref[1])
+
+
+def test_systems_of_different_size_on_two_threads():
+    """One thread solves a system of nearly 3 million values, whose iterations
+    take several launches of most of an SM's shared memory, while another
+    solves one of a few rows over and over: both as alone, bit for bit."""
+    import threading
+    from fea_b200 import _lib as L
+    P, K, b = system("C3D8", (23, 22, 22))
+    Q, K2, b2 = system("C3D8", (1, 1, 1), "roller")
+    assert 2_500_000 < P.nnz < 3_000_000 and Q.ndof < 24
+    ref = [torch.zeros_like(b), torch.zeros_like(b2)]
+    assert P.pcg(K, b, ref[0], 1e-300, 1000)[::2] == (1000, L.FEA_ENOTCONV)   # (about 190 iterations per launch)
+    assert Q.pcg(K2, b2, ref[1], 1e-20, 500)[2] == 0
+    torch.cuda.synchronize()
+    stop, count, errors = threading.Event(), [0], []
+
+    def small():
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                while not stop.is_set():
+                    x = torch.zeros_like(b2)
+                    Q.pcg(K2, b2, x, 1e-20, 500)
+                    assert torch.equal(x, ref[1])
+                    count[0] += 1
+        except BaseException as e:
+            errors.append(e)
+    th = threading.Thread(target=small)
+    th.start()
+    try:
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(6):
+                x = torch.zeros_like(b)
+                assert P.pcg(K, b, x, 1e-300, 1000)[::2] == (1000, L.FEA_ENOTCONV)
+                assert torch.equal(x, ref[0])
+    finally:
+        stop.set()
+        th.join()
+    assert not errors and count[0] > 0
