@@ -1008,8 +1008,10 @@ static unsigned persist_grid(int64_t n) {
 }
 
 // PCG on a matrix that fits the shared memory of the grid's CTAs; *fits = false
-// (and nothing done) when it does not: the largest share is known once
-// k_persist_plan has run, which systems that cannot fit are spared.
+// when it does not: the largest share is known once k_persist_plan has run,
+// which systems that cannot fit are spared.  Also false where the device refuses
+// the cooperative launch (fewer SMs for this context than it reports): x then
+// holds the *iters iterations done so far.
 static int pcg_persist(const NodeOp<double>& A, int64_t nnz, const double* b, double* x, double tol, int max_iter,
                        int check_every, const PcgWork& W, bool* fits, int* iters, double* relres, cudaStream_t s) {
   *fits = false;
@@ -1053,8 +1055,14 @@ static int pcg_persist(const NodeOp<double>& A, int64_t nnz, const double* b, do
     if (host[S_DONE] != 0.0 || it_done >= max_iter) break;
     P.iters = std::min(ce, max_iter - it_done);
     void* args[] = {&P};
-    if (cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_pcg_persist, dim3(G), dim3(PP_TPB), args, P.smem, s))
-      return (int)e;
+    if (cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_pcg_persist, dim3(G), dim3(PP_TPB), args, P.smem, s)) {
+      if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorLaunchOutOfResources && e != cudaErrorNotSupported)
+        return (int)e;
+      cudaGetLastError();
+      *fits = false;
+      *iters = it_done;
+      return 0;
+    }
     count_launch();
     it_done += P.iters;
   }
@@ -1687,7 +1695,11 @@ extern "C" int fea_pcg_solve_nodes(const fea_nodes_t* N, const int32_t* ix, cons
   bool fits = false;
   int it = 0;
   int r = pcg_persist(A, N->nnz, b, x, tol, max_iter, check_every, W, &fits, &it, relres, s);
-  if (!fits && r == 0) r = pcg_core(A, n, b, x, W, tol, max_iter, check_every, &it, relres, s);
+  if (!fits && r == 0) {
+    const int before = it;
+    r = pcg_core(A, n, b, x, W, tol, max_iter - before, check_every, &it, relres, s);
+    it += before;
+  }
   if (iters) *iters = it;
   return r;
 }
