@@ -79,39 +79,22 @@ struct PlainVec {
   __device__ __forceinline__ X operator()(int64_t j) const { return x[j]; }
 };
 template <class X>
-struct PairVec;
-template <>
-struct PairVec<double> {
-  const double2* __restrict__ zp;
-  const double* st;
-  double beta;
-  __device__ __forceinline__ void init() { beta = st[S_BETA]; }
-  __device__ __forceinline__ double operator()(int64_t j) const {
-    return of(zp[j]);
-  }
-  __device__ __forceinline__ double of(double2 t) const { return fma(beta, t.y, t.x); }
-};
-template <>
-struct PairVec<float> {
-  const float2* __restrict__ zp;
-  const double* st;
-  float bh, bl;                      // beta to 48 bits
-  __device__ __forceinline__ void init() {
-    const double b = st[S_BETA];
-    bh = (float)b;
-    bl = (float)(b - (double)bh);
-  }
-  __device__ __forceinline__ float operator()(int64_t j) const {
-    return of(zp[j]);
-  }
-  __device__ __forceinline__ float of(float2 t) const { return fmaf(bh, t.y, fmaf(bl, t.y, t.x)); }
-};
-template <class X>
 struct PairOf;
 template <>
 struct PairOf<double> { typedef double2 type; };
 template <>
 struct PairOf<float> { typedef float2 type; };
+// (p in FP64, rounded once: the bits that k_pcg_p leaves)
+template <class X>
+struct PairVec {
+  typedef typename PairOf<X>::type Pair;
+  const Pair* __restrict__ zp;
+  const double* st;
+  double beta;
+  __device__ __forceinline__ void init() { beta = st[S_BETA]; }
+  __device__ __forceinline__ X operator()(int64_t j) const { return of(zp[j]); }
+  __device__ __forceinline__ X of(Pair t) const { return (X)fma(beta, (double)t.y, (double)t.x); }
+};
 
 // block sum: warp shuffles, then the 8 warp sums in fixed order
 __device__ __forceinline__ double block_sum_w(double v, double* sh) {
@@ -938,8 +921,8 @@ static PcgWork carve(double* w, int64_t n) {
 // own: a pair is twice the gathered bytes, and once the rows' vectors crowd
 // the caches the SpMV loses more than the p kernel takes.  us per iteration,
 // pairs and arrays: FP64 38.8 and 39.9 at 202k rows (40^3 C3D8), 60.0 and 61.5
-// at 346k, 98.1 and 96.8 at 546k, 152 and 142 at 811k; FP32 27.4 and 29.1, 36.8
-// and 39.2, 57.7 and 62.9, 96.3 and 99.8 (larger ones not measured).
+// at 346k, 98.1 and 96.8 at 546k, 152 and 142 at 811k; FP32 28.9 and 29.1, 38.8
+// and 39.6, 60.5 and 63.4, 98.7 and 99.5, 137 and 137 at 1.15M (the same bits).
 constexpr int64_t PAIR_ROWS64 = 450000, PAIR_ROWS32 = 1000000;
 template <class X>
 static int form_for(int64_t n) {

@@ -77,3 +77,40 @@ def test_newton_mixed_mode_on_padded_layout(golden):
     gc = c.solver.solve()
     assert not isinstance(gc, bool)
     assert rel(gc, g["gc_converged"]) < 1e-8
+
+
+@pytest.mark.parametrize("copies", [2, 60])
+def test_search_direction_has_the_same_bits_at_every_size(copies):
+    """p = z + beta p is formed in FP64 and rounded once, in the SpMV's gather
+    (small systems) as in a kernel of its own (large ones): several copies of
+    one system side by side take the steps of the single one (every sum is the
+    copies' multiple up to its FP64 rounding), so that the FP32 iterates hold
+    the same bits but where 1e-16 in a scalar crosses a rounding boundary, 1e-8
+    of them per step."""
+    import ctypes as C
+    from fea_b200 import _lib as L
+    rng = np.random.default_rng(7)
+    n1 = 20000
+    d, b1 = 2.0 + rng.uniform(0.01, 1.0, n1), rng.normal(size=n1)
+
+    def solve(k):
+        n = k * n1
+        row = np.arange(n1)
+        cols = row[:, None] + np.array([-1, 0, 1])
+        ok = (cols >= 0) & (cols < n1)
+        vals = np.where(cols == row[:, None], d[:, None], -1.0)
+        ip = np.concatenate([[0], np.cumsum(np.tile(ok.sum(1), k))]).astype(np.int64)
+        ix = (cols[ok][None, :] + n1 * np.arange(k)[:, None]).reshape(-1).astype(np.int32)
+        v = torch.from_numpy(np.tile(vals[ok], k)).cuda()
+        ip, ix, b = torch.from_numpy(ip).cuda(), torch.from_numpy(ix).cuda(), torch.from_numpy(np.tile(b1, k)).cuda()
+        v32, x = v.float(), torch.zeros(n, dtype=torch.float64, device="cuda")
+        w = torch.empty(int(L.fea_pcg_mixed_work_len(n)), dtype=torch.float64, device="cuda")
+        it, out, rr = C.c_int32(0), C.c_int32(0), C.c_double(0)
+        st = L.fea_pcg_solve_mixed(n, ip.data_ptr(), ix.data_ptr(), v.data_ptr(), v32.data_ptr(), b.data_ptr(), x.data_ptr(),
+                                   1e-30, 0.0, 12, 12, w.data_ptr(), w.numel(), C.byref(it), C.byref(out), C.byref(rr),
+                                   torch.cuda.current_stream().cuda_stream)
+        assert st == L.FEA_ENOTCONV and it.value == 12
+        return x.view(k, n1)
+    one, many = solve(1), solve(copies)
+    assert float((one != 0).double().mean()) > 0.99
+    assert float((many != one).double().mean()) < 1e-5
