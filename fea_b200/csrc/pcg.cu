@@ -919,14 +919,24 @@ static PcgWork carve(double* w, int64_t n) {
 
 // Rows up to which p is formed in the gather (pairs); above, by a kernel of its
 // own: a pair is twice the gathered bytes, and once the rows' vectors crowd
-// the caches the SpMV loses more than the p kernel takes.  us per iteration,
-// pairs and arrays: FP64 38.8 and 39.9 at 202k rows (40^3 C3D8), 60.0 and 61.5
-// at 346k, 98.1 and 96.8 at 546k, 152 and 142 at 811k; FP32 28.9 and 29.1, 38.8
-// and 39.6, 60.5 and 63.4, 98.7 and 99.5, 137 and 137 at 1.15M (the same bits).
-constexpr int64_t PAIR_ROWS64 = 450000, PAIR_ROWS32 = 1000000;
-template <class X>
-static int form_for(int64_t n) {
-  return n <= (sizeof(X) == 8 ? PAIR_ROWS64 : PAIR_ROWS32) ? FORM_PAIRS : FORM_ARRAYS;
+// the caches the SpMV loses more than the p kernel takes; a kernel with one
+// gather per value and many of them in flight (the plain rows, the FP32 values
+// in the plan's layout) loses it earlier.  us per iteration, pairs and arrays, C3D8
+// blocks, at 45k, 105k, 202k, 346k, 546k, 811k and 1.15M rows:
+//   NodeOp<double>  16.9 18.2  25.9 28.4  39.0 40.5  58.8 60.2  97.1 95.6  142 139
+//   CsrOp<double>   19.7 20.6  35.6 37.5  62.0 62.3  98.2 98.4  147 147  212 211
+//   NodeOp32q       15.2 16.6  18.9 20.4  28.9 29.1  38.8 39.6  60.5 63.4  98.7 99.5  137 137
+//   NodeOp<float>   18.6 18.8 (71k: 21.7 21.6)  27.5 25.5  44.8 36.5  69.3 54.1  120 89  178 128
+//   CsrOp<float>    23.1 22.3 (26k: 17.6 17.7)  37.1 33.5  64.4 57.2  100 88.3  150 134  218 191
+// Both leave the same bits.
+template <class V>
+constexpr int64_t pair_rows(const CsrOp<V>&) { return sizeof(V) == 8 ? 450000 : 30000; }
+template <class V>
+constexpr int64_t pair_rows(const NodeOp<V>&) { return sizeof(V) == 8 ? 450000 : 60000; }
+constexpr int64_t pair_rows(const NodeOp32q&) { return 1000000; }
+template <class Op>
+static int form_for(const Op& A, int64_t n) {
+  return n <= pair_rows(A) ? FORM_PAIRS : FORM_ARRAYS;
 }
 
 // One iteration: q = A p with p.q and alpha; x, r, z with r.z, beta and the stop test
@@ -957,7 +967,7 @@ static int pcg_core(const Op& A, int64_t n, const double* b, double* x, const Pc
                     int check_every, int* iters, double* relres, cudaStream_t s) {
   spmv(A, (const double*)x, W.r, s);                      // r = A x
   const unsigned vg = vec_grid<double>(n);
-  const int form = form_for<double>(n);
+  const int form = form_for(A, n);
   k_pcg_setup<double><<<vg, PCG_TPB, 0, s>>>(n, b, W.r, W.zp, W.dinv, W.st, W.part, W.counter, form, nullptr);
   count_launch();
   if (cudaError_t e = cudaGetLastError()) return (int)e;
@@ -1109,7 +1119,7 @@ static int pcg_mixed(const Op64& A, const Op32& A32, int64_t n, const double* b,
     // FP32 start from r64: x32 = 0, r32 = r64, z32, p32, rho; stop test scale from b
     cudaMemsetAsync(xf, 0, sizeof(float) * n, s);
     cudaMemsetAsync(rf, 0, sizeof(float) * n, s);
-    const int form = form_for<float>(n);
+    const int form = form_for(A32, n);
     k_pcg_setup<float><<<vgf, PCG_TPB, 0, s>>>(n, W.r, rf, zpf, W.dinv, st2, W.part, counter2, form, nullptr);
     count_launch();
     cudaMemcpyAsync(st2 + S_RZ0, W.st + S_RZ0, sizeof(double), cudaMemcpyDeviceToDevice, s);
