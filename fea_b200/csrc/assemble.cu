@@ -308,8 +308,7 @@ __device__ __forceinline__ void tet_strip(const VolParams& P, const int32_t cn[4
 #pragma unroll
     for (int i = 0; i < 3; ++i)
       F[3 * I + i] = fma(Ju[3 * I], iJ[i], fma(Ju[3 * I + 1], iJ[3 + i], fma(Ju[3 * I + 2], iJ[6 + i], I == i ? 1.0 : 0.0)));
-  double Jm;
-  const double J = inv3_jm(F, iF, &Jm);
+  const double J = inv3(F, iF), Jm = jm23(J);
   const double mu = P.mu, kappa = P.kappa;
   double sF2 = 0.0;
 #pragma unroll

@@ -3,8 +3,8 @@ kernel, which the same entry point takes for a descriptor without lists:
 chunks with one and with many nodes, a node shared by 120 tetrahedra, partly
 fixed nodes, a doubled element, accumulate, no residual, and the
 element residual.  Each entry sums the same contributions in the same order;
-the strips differ by the rounding of 1/J (three roundings instead of a
-division) and of g_a . g_b: 1e-12 of the largest entry bounds it."""
+the strips differ by the rounding of g_a . g_b (formed as f_a . q_b): 1e-12 of the
+largest entry bounds it."""
 import ctypes as C
 
 import numpy as np
@@ -78,6 +78,62 @@ def test_lists_match_rank_rounds(kind, repeat):
                     out.append((pad, R, eR))
                 for a, b in zip(*out):
                     assert float((a - b).abs().max()) <= TOL * max(1.0, float(a.abs().max()))
+
+
+def tangent80(X, el, u, mu, kappa):
+    """Element tangents [E, 12, 12] in 80-bit arithmetic."""
+    T = np.longdouble
+    d = np.array([[-1, -1, -1], [1, 0, 0], [0, 1, 0], [0, 0, 1]], T)
+
+    def inv(m):
+        c = np.stack([np.cross(m[:, 1], m[:, 2]), np.cross(m[:, 2], m[:, 0]), np.cross(m[:, 0], m[:, 1])], 2)
+        det = (m[:, 0] * c[:, :, 0]).sum(1)
+        return c / det[:, None, None], det
+    iJ, det = inv(np.einsum("bm,ebi->eim", d, X.astype(T)[el]))
+    g = np.einsum("bm,emi->ebi", d, iJ)
+    F = np.eye(3, dtype=T) + np.einsum("ebk,ebi->eki", u.astype(T)[el], g)
+    iF, J = inv(F)
+    c = mu * np.exp(-2 * np.log(J) / 3)
+    I1m = c * (F * F).sum((1, 2))
+    q, f = np.einsum("eik,ebi->ebk", iF, g), np.einsum("eki,ebi->ebk", F, g)
+    mul = lambda s, a, b, o: np.einsum("e,eaj,ebk->" + o, s * det / 6, a, b)  # noqa: E731
+    K = mul(-2 * c / 3, f, q, "eajbk") + mul(-2 * c / 3, q, f, "eajbk")
+    K += mul(kappa * J * (2 * J - 1) + 2 * I1m / 9, q, q, "eajbk") + mul(I1m / 3 - kappa * J * (J - 1), q, q, "eakbj")
+    K += np.einsum("e,eai,ebi,jk->eajbk", c * det / 6, g, g, np.eye(3, dtype=T))
+    return K.reshape(len(el), 12, 12)
+
+
+@gpu
+@pytest.mark.parametrize("dims", [(5, 4, 3), (9, 8, 7)])
+def test_tangent_error_is_that_of_the_rank_rounds(dims):
+    """Against the element tangents in 80 bits, K by lists is no further off
+    than K in rank rounds (2.6e-16 relative, of which the last bits of the
+    sums alone make 2 percent either way; 1/J by a cube in place of a division 11 to
+    16 percent more)."""
+    from fea_b200 import DevicePlan
+    from fea_b200 import _lib as L
+    X, el = mesh(dims)
+    P = DevicePlan(X, np.full(len(X), 7, np.uint8), [("C3D4", el)])
+    g = P.groups[0]
+    u = np.random.default_rng(4).normal(0, 0.02 / max(dims), X.shape)
+    dof = (3 * el[:, :, None] + np.arange(3)).reshape(len(el), 12)
+    n = P.ndof
+    ip, ix = P.indptr.cpu().numpy(), P.indices.cpu().numpy()
+    key = np.repeat(np.arange(n), np.diff(ip)) * n + ix
+    ref = np.zeros(P.nnz, np.longdouble)
+    np.add.at(ref, np.searchsorted(key, dof[:, :, None] * n + dof[:, None, :]), tangent80(X, el, u, 1.0, 20.0))
+    old = L.Group()
+    C.memmove(C.byref(old), C.byref(g.desc), C.sizeof(L.Group))
+    old.clist_dev = None
+    gc = torch.from_numpy(u.reshape(-1)).cuda()
+    err = []
+    for d in (old, g.desc):
+        K = torch.empty(P.nnz, dtype=torch.float64, device="cuda")
+        L.check(L.fea_assemble_volume(C.byref(P.nodes), C.byref(d), 1.0, 20.0, ptr(gc), ptr(K), None, None, 0, None, 0,
+                                      C.c_void_p(torch.cuda.current_stream().cuda_stream)), "tet")
+        e = K.cpu().numpy().astype(np.longdouble) - ref
+        err.append(float(np.sqrt((e * e).sum() / (ref * ref).sum())))
+    assert 1e-17 < err[0] < 1e-15 and err[1] <= 1.04 * err[0], err
 
 
 def test_lists_of_the_host_plan():
