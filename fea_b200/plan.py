@@ -474,7 +474,11 @@ class DevicePlan:
                                      vptr(vhp), vptr(a), vptr(v), stream()), "fea_explicit_stage")
 
     def explicit_run(self, gi, mu, kappa, minv, dt, steps, u, vh, a, v, fp32=False, init=False):
-        w = self.scratch(L.fea_explicit_group_work_len(C.byref(self.nodes), C.byref(self.groups[gi].desc)))
+        n = int(L.fea_explicit_group_work_len(C.byref(self.nodes), C.byref(self.groups[gi].desc)))
+        try:
+            w = torch.empty(n, dtype=torch.float64, device=self.device)
+        except torch.cuda.OutOfMemoryError:       # without the elements' parts every node evaluates its elements
+            w = self.scratch(L.fea_explicit_work_len(C.byref(self.nodes)))
         L.check(L.fea_explicit_run(C.byref(self.nodes), C.byref(self.groups[gi].desc), float(mu), float(kappa),
                                    vptr(minv), float(dt), int(steps), int(bool(fp32)), int(bool(init)), vptr(u),
                                    vptr(vh), vptr(a), vptr(v), vptr(w), w.numel(), stream()), "fea_explicit_run")

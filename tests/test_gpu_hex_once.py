@@ -180,6 +180,38 @@ def test_explicit_steps(dims, fp32):
         assert float((x - y).abs().max()) <= tol * float(x.abs().max())
 
 
+@pytest.mark.parametrize("kind", ["C3D8", "C3D4"])
+def test_explicit_run_where_the_long_buffer_does_not_fit(kind, monkeypatch):
+    """Without memory for the elements' parts DevicePlan.explicit_run takes the
+    per-node path, as it did before it had another."""
+    from fea_b200 import DevicePlan
+    from fea_b200 import _lib as L
+    from fea_b200.meshes import hex_block, tet_block
+    X, el = (hex_block if kind == "C3D8" else tet_block)(0, dims=(9, 8, 7))
+    P = DevicePlan(X, np.full(len(X), 7, np.uint8), [(kind, el)])
+    u0 = 1e-3 * torch.randn(P.ndof, dtype=torch.float64, generator=torch.Generator().manual_seed(5)).cuda()
+    minv = P.lumped_mass_inv([1.0])
+    short = int(L.fea_explicit_work_len(C.byref(P.nodes)))
+    assert int(L.fea_explicit_group_work_len(C.byref(P.nodes), C.byref(P.groups[0].desc))) > short > P.ndof
+    empty = torch.empty
+
+    def no_room(n, *a, **k):
+        if n > short:
+            raise torch.cuda.OutOfMemoryError("no room for %d" % n)
+        return empty(n, *a, **k)
+    out = []
+    for tight in (True, False):                   # (first without room: nothing may be kept from an earlier call)
+        u, v = u0.clone(), torch.zeros_like(u0)
+        vh, a = torch.zeros_like(u0), torch.zeros_like(u0)
+        with monkeypatch.context() as m:
+            if tight:
+                m.setattr(torch, "empty", no_room)
+            P.explicit_run(0, 1.0, 40.0, minv, 1e-3, 4, u, vh, a, v, init=True)
+        out.append((u, v, a))
+    for x, y in zip(*out):
+        assert not torch.equal(x, u0) and float((x - y).abs().max()) <= 10 * TOL * float(x.abs().max())
+
+
 @pytest.mark.parametrize("dims", MESHES + [(13, 8, 11), (12, 11, 12), (14, 13, 13)])
 @pytest.mark.parametrize("repeat", [False, True])
 def test_tangent_and_residual(dims, repeat):
