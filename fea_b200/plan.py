@@ -8,9 +8,7 @@ only launches kernels on the current torch stream.
 """
 from __future__ import annotations
 
-import contextlib
 import ctypes as C
-import threading
 
 import numpy as np
 import torch
@@ -19,9 +17,6 @@ from . import _lib as L
 
 KIND = {"C3D4": L.FEA_C3D4, "C3D8": L.FEA_C3D8, "T3": L.FEA_T3, "Q4": L.FEA_Q4}
 NODES_PER = {L.FEA_C3D4: 4, L.FEA_C3D8: 8, L.FEA_T3: 3, L.FEA_Q4: 4}
-
-
-_NO_LOCK = contextlib.nullcontext()
 
 
 def vptr(t):
@@ -172,8 +167,10 @@ class GatherGroup:
                               if self.lists else []))
         self.nchunk = int(self.desc.nchunk)
         # doubles of the element-once kernels' slots (C3D8 elements)
-        self.slot_len = (max(int(L.fea_force_work_len(C.byref(self.desc))), int(L.fea_adjoint_work_len(C.byref(self.desc))))
-                         if base == L.G_BASE and kind == L.FEA_C3D8 and self.ne else 0)
+        self.once = base == L.G_BASE and kind == L.FEA_C3D8 and self.ne > 0
+        if self.once:
+            self.force_len = int(L.fea_force_work_len(C.byref(self.desc)))
+            self.vjp_len = int(L.fea_adjoint_work_len(C.byref(self.desc)))
 
 
 class DevicePlan:
@@ -215,13 +212,6 @@ class DevicePlan:
                                  self.adjoff.data_ptr(), self.moff.data_ptr())
             self.groups = [GatherGroup(hp, L.G_BASE, i, k, c, self.device) for i, (k, c) in enumerate(gl)]
             self.faces = [GatherGroup(hp, L.F_BASE, i, k, c, self.device) for i, (k, c) in enumerate(fl)]
-            # slots of the element-once kernels (C3D8 residual, adjoint):
-            # laid out here, so that a first call does not wait for them
-            self._slots_len = max([g.slot_len for g in self.groups], default=0)
-            self._slots = (torch.empty(self._slots_len, dtype=torch.float64, device=self.device)
-                           if self._slots_len else None)
-            self._slots_stream = stream()
-            self._slots_lock = threading.Lock()
         self._scratch = None
         self._coo = None
 
@@ -254,20 +244,14 @@ class DevicePlan:
         return g._stage, n
 
     def slots(self, n):
-        """(buffer, n, lock): n doubles for the per-element slots of one call,
-        the lock held around its launches; (None, 0, ...) where there is no
-        memory for them (the entry points then take the path that needs
-        none).  Calls on the stream the plan was built on share the buffer
-        laid out with the plan, one call's launches at a time (launches of two
-        host threads do not interleave, and the stream orders them); calls on
-        other streams, or under capture, take a buffer of their own from the
-        caching allocator."""
-        if n <= self._slots_len and stream() == self._slots_stream and not torch.cuda.is_current_stream_capturing():
-            return self._slots, n, self._slots_lock
+        """n doubles for the per-element slots of one call, from the caching
+        allocator (of the calling stream, or of a capture's pool), or None
+        where there is no memory for them: the entry points then take the
+        path that needs none."""
         try:
-            return torch.empty(n, dtype=torch.float64, device=self.device), n, _NO_LOCK
+            return torch.empty(n, dtype=torch.float64, device=self.device)
         except torch.cuda.OutOfMemoryError:
-            return None, 0, _NO_LOCK
+            return None
 
     def assemble_volume(self, gi, mu, kappa, gc, K=None, R=None, elemR=None, accumulate=False):
         g = self.groups[gi]
@@ -275,14 +259,10 @@ class DevicePlan:
         need(K, self.nnz, self.device, "K")
         need(R, self.ndof, self.device, "R")
         need(elemR, g.nn * 3 * g.ne, self.device, "elemR")
-        if K is not None or g.slot_len == 0:
-            (w, wn), lock = self.stage(gi) if K is not None else (None, 0), _NO_LOCK
-        else:
-            w, wn, lock = self.slots(g.slot_len)
-        with lock:
-            L.check(L.fea_assemble_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
-                                          vptr(K), vptr(R), vptr(elemR), int(bool(accumulate)), vptr(w), int(wn),
-                                          stream()), "fea_assemble_volume")
+        w = self.stage(gi)[0] if K is not None else self.slots(g.force_len) if g.once else None
+        L.check(L.fea_assemble_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
+                                      vptr(K), vptr(R), vptr(elemR), int(bool(accumulate)), vptr(w),
+                                      w.numel() if w is not None else 0, stream()), "fea_assemble_volume")
 
     def assemble_pressure(self, fi, p, Xinst, gc, K=None, R=None):
         f = self.faces[fi]
@@ -335,14 +315,12 @@ class DevicePlan:
     def adjoint_vjp_volume(self, gi, mu, kappa, gc, lam_full, dX, dmu):
         """dX += d(lam . R_e)/dX (all nodes); dmu[0] = d(lam . R_e)/dmu."""
         g = self.groups[gi]
-        s, n, lock = self.slots(g.slot_len) if g.slot_len else (None, 0, _NO_LOCK)
+        s = self.slots(g.vjp_len) if g.once else None
         if s is None:
             s = self.scratch(L.fea_reduce_scratch_len(g.ne))
-            n = s.numel()
-        with lock:
-            L.check(L.fea_adjoint_vjp_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
-                                             vptr(lam_full), vptr(dX), vptr(dmu), vptr(s), int(n), stream()),
-                    "fea_adjoint_vjp_volume")
+        L.check(L.fea_adjoint_vjp_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
+                                         vptr(lam_full), vptr(dX), vptr(dmu), vptr(s), s.numel(), stream()),
+                "fea_adjoint_vjp_volume")
 
     def adjoint_hvp_pressure(self, fi, p, Xinst, gc, v_full, out):
         """out += p d2V/dx2 v (all nodes) for face group fi."""

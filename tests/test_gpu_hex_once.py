@@ -88,8 +88,8 @@ def test_residual(dims, acc, repeat):
 
 
 def test_residual_on_streams_and_under_capture():
-    """The plan's own buffer serves its own stream; other streams and a
-    capture take their own, with the same bits."""
+    """Every call takes its slots from the allocator of its stream or of the
+    capture, with the same bits."""
     P, gc = hex_plan((6, 5, 4))
     ref = P.zeros(P.ndof)
     P.assemble_volume(0, 1.0, 40.0, gc, R=ref)
@@ -178,6 +178,47 @@ def test_explicit_steps(dims, fp32):
     tol = 1e-4 if fp32 else TOL * 10
     for x, y in zip(*out):
         assert float((x - y).abs().max()) <= tol * float(x.abs().max())
+
+
+def test_plans_hold_no_slots(monkeypatch):
+    """The slots live for one call: neither a new plan nor one that has
+    computed residuals and gradients holds them, and without memory for them
+    the general path gives the same."""
+    from fea_b200 import DevicePlan
+    from fea_b200.meshes import hex_block
+    X, el = hex_block(0, dims=(24, 24, 24))
+
+    def plan():
+        return DevicePlan(X, np.full(len(X), 7, np.uint8), [("C3D8", el)])
+    P = plan()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    Q = plan()
+    held = torch.cuda.memory_allocated() - before
+    arrays = sum(t.numel() * t.element_size() for o in (Q, Q.groups[0]) for t in vars(o).values() if isinstance(t, torch.Tensor))
+    slots = 8 * 32 * len(el)
+    assert arrays <= held < arrays + slots / 4
+    gc = 1e-3 * torch.randn(P.ndof, dtype=torch.float64, generator=torch.Generator().manual_seed(5)).cuda()
+    lam = torch.randn(P.n_nodes, 3, dtype=torch.float64, generator=torch.Generator().manual_seed(4)).cuda()
+    out, empty = [], torch.empty
+
+    def no_room(n, *a, **k):
+        if n >= slots / 8:
+            raise torch.cuda.OutOfMemoryError("no room for %d" % n)
+        return empty(n, *a, **k)
+    for tight in (True, False):
+        R, dX, dmu = P.zeros(P.ndof), torch.zeros_like(lam), P.zeros(1)
+        before = torch.cuda.memory_allocated()
+        with monkeypatch.context() as m:
+            if tight:
+                m.setattr(torch, "empty", no_room)
+            P.assemble_volume(0, 1.0, 40.0, gc, R=R)
+            P.adjoint_vjp_volume(0, 1.0, 40.0, gc, lam, dX, dmu)
+        assert torch.cuda.memory_allocated() - before < slots / 4
+        out.append((R, dX))
+    assert not torch.equal(*[o[0] for o in out])  # two paths, to rounding the same
+    for x, y in zip(*out):
+        assert close(x, y)
 
 
 @pytest.mark.parametrize("kind", ["C3D8", "C3D4"])
