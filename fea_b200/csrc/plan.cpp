@@ -55,9 +55,7 @@ struct GatherList {            // one element group or one face group
   std::vector<int32_t> stagepos;   // [ne*36] staged block of each element block (lane slot order), -1: none
   std::vector<int64_t> region;     // [N+1] first staged block of each node's region (even)
   int32_t hx_stride = 0;           // C3D8: regions at n * hx_stride, 16 records per node (0: by region / uptr)
-  std::vector<uint16_t> clist;     // [ninc*4] C3D4: a node's contributions column by column (TET_* codes)
-  std::vector<uint32_t> crec;      // 2 per neighbour of a node (itself first): offset | mask << 16, start | count << 11
-  std::vector<int64_t> crecptr;    // [N+1] first neighbour record of each node
+  std::vector<int64_t> crecptr;    // [N+1] C3D4: first neighbour record of each node
   std::vector<int32_t> tileptr;    // [ntile+1] into chunklist: C3D4 tiles
   std::vector<int32_t> allptr;     // [N+1] incidences of every node (constrained ones included)
   std::vector<int32_t> allinc;     // e*16 + a, element order ascending
@@ -215,51 +213,13 @@ int build_gather(const fea_plan& P, int kind, int64_t ne, const int32_t* conn, c
   return FEA_OK;
 }
 
-// Neighbour lists of a C3D4 group.  Incidence r of a row node holds 4 blocks
-// of 9 values and the 3 of the residual (FEA_TET_STRIDE doubles in the
-// kernel's shared memory); clist lists the offsets (r * stride + 9 b) of the
-// blocks that fall on each neighbour, neighbour by neighbour, in incidence
-// order.  The neighbours' records, the node itself first, say where the
-// neighbour's columns are in the node's rows (offset, free components) and
-// which part of the list is its (start, count).
-void build_tet_lists(const fea_plan& P, const int32_t* conn, const Incidence& I, GatherList& G) {
+// Places of a C3D4 group's neighbour records (the lists are made when asked
+// for: tet_lists here, fea_tet_lists on the device) and its tiles.
+void build_tet_tiles(const fea_plan& P, GatherList& G) {
   const int64_t N = P.N;
   G.crecptr.assign(N + 1, 0);
   for (int64_t n = 0; n < N; ++n)
     G.crecptr[n + 1] = G.crecptr[n] + (G.nodeinc[n + 1] > G.nodeinc[n] ? P.adjptr[n + 1] - P.adjptr[n] : 0);
-  G.crec.assign((size_t)G.crecptr[N] * 2, 0);
-  G.clist.assign((size_t)G.nodeinc[N] * 4, 0);
-  parallel_for(N, [&](int64_t a0, int64_t a1) {
-    std::vector<int32_t> at, slot;
-    for (int64_t n = a0; n < a1; ++n) {
-      const int64_t ni = G.nodeinc[n + 1] - G.nodeinc[n];
-      if (ni == 0) continue;
-      const int64_t p0 = P.adjptr[n], np = P.adjptr[n + 1] - p0;
-      const int32_t* col = P.adjcol.data() + p0;
-      at.assign(np + 1, 0);
-      slot.assign(ni * 4, -1);
-      for (int64_t r = 0; r < ni; ++r) {
-        const int64_t e = I.ent[I.ptr[n] + r] >> 4;
-        for (int b = 0; b < 4; ++b) {
-          const int32_t c = conn[e * 4 + b];
-          if (!P.mask[c]) continue;
-          slot[r * 4 + b] = (int32_t)(std::lower_bound(col, col + np, c) - col);
-          at[slot[r * 4 + b] + 1]++;
-        }
-      }
-      const int64_t self = std::lower_bound(col, col + np, (int32_t)n) - col;
-      for (int64_t k = 0; k < np; ++k) {
-        const int64_t u = G.crecptr[n] + (k == self ? 0 : k < self ? k + 1 : k);
-        G.crec[2 * u] = (uint32_t)P.adjoff[p0 + k] | (uint32_t)P.mask[col[k]] << 16;
-        G.crec[2 * u + 1] = (uint32_t)at[k] | (uint32_t)at[k + 1] << 11;   // (at[k + 1] still a count)
-        at[k + 1] += at[k];
-      }
-      for (int64_t r = 0; r < ni; ++r)
-        for (int b = 0; b < 4; ++b)
-          if (slot[r * 4 + b] >= 0)
-            G.clist[(size_t)G.nodeinc[n] * 4 + at[slot[r * 4 + b]]++] = (uint16_t)(r * FEA_TET_STRIDE + 9 * b);
-    }
-  });
   // tiles of consecutive nodes with at most FEA_TET_TILE incidences
   G.tileptr.assign(1, 0);
   for (size_t l = 0, i0 = 0; l < G.chunklist.size(); ++l) {
@@ -270,6 +230,45 @@ void build_tet_lists(const fea_plan& P, const int32_t* conn, const Incidence& I,
     }
   }
   if (!G.chunklist.empty()) G.tileptr.push_back((int32_t)G.chunklist.size());
+}
+
+// Neighbour lists of a C3D4 group.  Incidence r of a row node holds 4 blocks
+// of 9 values and the 3 of the residual (FEA_TET_STRIDE doubles in the
+// kernel's shared memory); clist [ninc*4] lists the offsets (r * stride + 9 b) of
+// the blocks that fall on each neighbour, neighbour by neighbour, in incidence
+// order.  The neighbours' records, the node itself first, say where the
+// neighbour's columns are in the node's rows (offset, free components) and
+// which part of the list is its (start, count).  Either may be NULL.
+void tet_lists(const fea_plan& P, const GatherList& G, uint16_t* clist, uint32_t* crec) {
+  if (clist) std::fill(clist, clist + (size_t)G.nodeinc[P.N] * 4, (uint16_t)0);
+  parallel_for(P.N, [&](int64_t a0, int64_t a1) {
+    std::vector<int32_t> at, slot;
+    for (int64_t n = a0; n < a1; ++n) {
+      const int64_t nc = 4 * (int64_t)(G.nodeinc[n + 1] - G.nodeinc[n]);
+      if (nc == 0) continue;
+      const int64_t p0 = P.adjptr[n], np = P.adjptr[n + 1] - p0;
+      const int32_t *col = P.adjcol.data() + p0, *off = P.adjoff.data() + p0;
+      const uint16_t* bo = G.boff.data() + 4 * (int64_t)G.nodeinc[n];
+      at.assign(np + 1, 0);
+      slot.assign(nc, -1);
+      for (int64_t t = 0; t < nc; ++t) {
+        if (bo[t] == 0xFFFF) continue;
+        slot[t] = (int32_t)(std::lower_bound(off, off + np, (int32_t)bo[t]) - off);
+        at[slot[t] + 1]++;
+      }
+      const int64_t self = std::lower_bound(col, col + np, (int32_t)n) - col;
+      for (int64_t k = 0; k < np; ++k) {
+        const int64_t u = G.crecptr[n] + (k == self ? 0 : k < self ? k + 1 : k);
+        if (crec) {
+          crec[2 * u] = (uint32_t)off[k] | (uint32_t)P.mask[col[k]] << 16;
+          crec[2 * u + 1] = (uint32_t)at[k] | (uint32_t)at[k + 1] << 11;   // (at[k + 1] still a count)
+        }
+        at[k + 1] += at[k];
+      }
+      for (int64_t t = 0; clist && t < nc; ++t)
+        if (slot[t] >= 0) clist[4 * (int64_t)G.nodeinc[n] + at[slot[t]]++] = (uint16_t)((t >> 2) * FEA_TET_STRIDE + 9 * (t & 3));
+    }
+  });
 }
 
 // Staging of a C3D8 group.  An element block couples the unordered local
@@ -542,7 +541,7 @@ extern "C" int fea_plan_build(int64_t n_nodes, const uint8_t* free_mask, int32_t
     if (r) return r;
     // (a node of more incidences than a tile holds: no lists, rank rounds)
     if (group_kind[g] == FEA_C3D4 && P->groups[g].maxval <= FEA_TET_TILE)
-      build_tet_lists(*P, group_conn[g], ginc[g], P->groups[g]);
+      build_tet_tiles(*P, P->groups[g]);
     if (group_kind[g] == FEA_C3D8 && (r = build_blocks(*P, 8, group_conn[g], ginc[g], P->groups[g]))) return r;
   }
   for (int g = 0; g < n_faces; ++g) {
@@ -613,8 +612,12 @@ extern "C" int fea_plan_get(const fea_plan* P, int32_t id, int32_t group, void* 
       case 18: return put(G->stagepos, dst, count);
       case 19: return put(G->region, dst, count);
       case 20: return scalar(G->hx_stride, count);
-      case 21: return put(G->clist, dst, count);
-      case 22: return put(G->crec, dst, count);
+      case 21:
+      case 22:
+        if (count) *count = G->crecptr.empty() ? 0 : id == 21 ? (int64_t)G->nodeinc[P->N] * 4 : G->crecptr[P->N] * 2;
+        if (dst && !G->crecptr.empty())
+          tet_lists(*P, *G, id == 21 ? static_cast<uint16_t*>(dst) : nullptr, id == 22 ? static_cast<uint32_t*>(dst) : nullptr);
+        return FEA_OK;
       case 23: return put(G->crecptr, dst, count);
       case 24: return put(G->tileptr, dst, count);
       default: return FEA_EINVAL;

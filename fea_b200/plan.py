@@ -9,6 +9,7 @@ only launches kernels on the current torch stream.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 import torch
@@ -139,12 +140,13 @@ class GatherGroup:
         self.region = dev(region) if uptr.size else None
         nblk = int(region[-1])
         maxblk = int(np.diff(region).max()) if region.size > 1 else 0
-        # neighbour lists of a C3D4 group (bit patterns: torch has no plain unsigned types)
-        self.lists = []
-        if base == L.G_BASE and hp.array(L.FEA_A_G_CRECPTR, index).size:
-            self.lists = [dev(hp.array(aid, index).view(vt)) for aid, vt in
-                          ((L.FEA_A_G_CLIST, np.int16), (L.FEA_A_G_CREC, np.int32), (L.FEA_A_G_CRECPTR, np.int64),
-                           (L.FEA_A_G_TILEPTR, np.int32))]
+        # C3D4: places of the tangent's neighbour records and its tiles (the
+        # lists themselves with the first tangent, DevicePlan.tangent_lists)
+        self.crecptr = self.tileptr = self.lists = None
+        crecptr = hp.array(L.FEA_A_G_CRECPTR, index) if base == L.G_BASE else np.zeros(0, np.int64)
+        if crecptr.size and nodeinc[-1] > 0:
+            self.crecptr, self.tileptr = dev(crecptr), dev(hp.array(L.FEA_A_G_TILEPTR, index))
+            self.ninc, self.nrec = int(nodeinc[-1]), int(crecptr[-1])
         self.allptr = dev(hp.array(base + L.A_ALLPTR, index))
         self.allinc = dev(hp.array(base + L.A_ALLINC, index))
         self.ne = int(self.conn.shape[0])
@@ -163,8 +165,8 @@ class GatherGroup:
                             self.stagepos.data_ptr() if self.stagepos is not None else None,
                             self.region.data_ptr() if self.region is not None else None, nblk, maxblk,
                             hp.scalar(L.FEA_S_G_HXSTRIDE, index) if uptr.size else 0,
-                            *([t.data_ptr() for t in self.lists] + [self.lists[-1].numel() - 1]
-                              if self.lists else []))
+                            *((None, None, self.crecptr.data_ptr(), self.tileptr.data_ptr(), self.tileptr.numel() - 1)
+                              if self.crecptr is not None else ()))
         self.nchunk = int(self.desc.nchunk)
         # doubles of the element-once kernels' slots (C3D8 elements)
         self.once = base == L.G_BASE and kind == L.FEA_C3D8 and self.ne > 0
@@ -212,6 +214,7 @@ class DevicePlan:
                                  self.adjoff.data_ptr(), self.moff.data_ptr())
             self.groups = [GatherGroup(hp, L.G_BASE, i, k, c, self.device) for i, (k, c) in enumerate(gl)]
             self.faces = [GatherGroup(hp, L.F_BASE, i, k, c, self.device) for i, (k, c) in enumerate(fl)]
+        self._lists_lock = threading.Lock()
         self._scratch = None
         self._coo = None
 
@@ -243,6 +246,35 @@ class DevicePlan:
             g._stage = torch.empty(n, dtype=torch.float64, device=self.device)
         return g._stage, n
 
+    def tangent_lists(self, gi):
+        """(descriptor, buffers) of group gi for a tangent: a C3D4 group's with
+        its neighbour lists (fea_tet_lists), made on the device with the
+        group's first tangent and kept; any other group's as it is.  The
+        first caller waits for them, so that every stream may use them.  A
+        capture that comes first takes lists of its own, made anew by each
+        replay.  Without memory for them the tangent is summed in rank
+        rounds."""
+        g = self.groups[gi]
+        if g.crecptr is None or g.lists is not None:
+            return g.desc, None
+        with self._lists_lock:
+            if g.lists is not None:
+                return g.desc, None
+            try:
+                clist = torch.empty(4 * g.ninc, dtype=torch.int16, device=self.device)
+                crec = torch.empty(2 * g.nrec, dtype=torch.int32, device=self.device)
+            except torch.cuda.OutOfMemoryError:
+                return g.desc, None
+            L.check(L.fea_tet_lists(C.byref(self.nodes), C.byref(g.desc), vptr(clist), vptr(crec), stream()), "fea_tet_lists")
+            if torch.cuda.is_current_stream_capturing():
+                d = L.Group.from_buffer_copy(g.desc)
+                d.clist_dev, d.crec_dev = vptr(clist), vptr(crec)
+                return d, (clist, crec)
+            torch.cuda.current_stream().synchronize()
+            g.desc.clist_dev, g.desc.crec_dev = vptr(clist), vptr(crec)
+            g.lists = (clist, crec)
+        return g.desc, None
+
     def slots(self, n):
         """n doubles for the per-element slots of one call, from the caching
         allocator (of the calling stream, or of a capture's pool), or None
@@ -259,8 +291,9 @@ class DevicePlan:
         need(K, self.nnz, self.device, "K")
         need(R, self.ndof, self.device, "R")
         need(elemR, g.nn * 3 * g.ne, self.device, "elemR")
+        d, keep = self.tangent_lists(gi) if K is not None else (g.desc, None)
         w = self.stage(gi)[0] if K is not None else self.slots(g.force_len) if g.once else None
-        L.check(L.fea_assemble_volume(C.byref(self.nodes), C.byref(g.desc), float(mu), float(kappa), vptr(gc),
+        L.check(L.fea_assemble_volume(C.byref(self.nodes), C.byref(d), float(mu), float(kappa), vptr(gc),
                                       vptr(K), vptr(R), vptr(elemR), int(bool(accumulate)), vptr(w),
                                       w.numel() if w is not None else 0, stream()), "fea_assemble_volume")
 

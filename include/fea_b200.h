@@ -232,12 +232,19 @@ typedef struct {
                                  the fixed layout (regions at n * hx_stride =
                                  n * maxblk, records at 16 n, residual slots at
                                  n * maxval); 0: packed (REGION, UPTR, NODEINC) */
-  const uint16_t* clist_dev;  /* FEA_A_G_CLIST, _CREC, _CRECPTR, _TILEPTR     */
-  const uint32_t* crec_dev;   /* (C3D4 only); any NULL: the tangent is summed */
-  const int64_t* crecptr_dev; /* in rank rounds                               */
+  const uint16_t* clist_dev;  /* FEA_A_G_CLIST, _CREC (or fea_tet_lists),     */
+  const uint32_t* crec_dev;   /* _CRECPTR, _TILEPTR (C3D4 only); any NULL:    */
+  const int64_t* crecptr_dev; /* the tangent is summed in rank rounds         */
   const int32_t* tileptr_dev;
   int64_t ntile;
 } fea_group_t;
+
+/* CLIST and CREC of a C3D4 group written on the device, from its boff_dev,
+ * nodeinc_dev and crecptr_dev (the same bits as the plan's arrays): clist_dev
+ * [ninc*4], crec_dev [2 * crecptr[N]], 8-byte aligned.  FEA_ECHUNK when a node has
+ * more than FEA_TET_TILE incidences (no lists, no CRECPTR). */
+int fea_tet_lists(const fea_nodes_t* nodes, const fea_group_t* group, uint16_t* clist_dev, uint32_t* crec_dev,
+                  cudaStream_t stream);
 
 /* Element residual and tangent of one Neo-Hookean group, gathered per node
  * row and written once into the reduced CSR values (store mode) or added to

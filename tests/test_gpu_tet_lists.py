@@ -60,6 +60,7 @@ def test_lists_match_rank_rounds(kind, repeat):
     g = P.groups[0]
     gc = torch.from_numpy(np.random.default_rng(2).normal(0, 5e-3 / (1 if kind == "fan" else max(kind)), P.ndof)).cuda()
     st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert P.tangent_lists(0)[0].clist_dev
     old = L.Group()
     C.memmove(C.byref(old), C.byref(g.desc), C.sizeof(L.Group))
     old.clist_dev = None
@@ -122,6 +123,7 @@ def test_tangent_error_is_that_of_the_rank_rounds(dims):
     key = np.repeat(np.arange(n), np.diff(ip)) * n + ix
     ref = np.zeros(P.nnz, np.longdouble)
     np.add.at(ref, np.searchsorted(key, dof[:, :, None] * n + dof[:, None, :]), tangent80(X, el, u, 1.0, 20.0))
+    assert P.tangent_lists(0)[0].clist_dev
     old = L.Group()
     C.memmove(C.byref(old), C.byref(g.desc), C.sizeof(L.Group))
     old.clist_dev = None
@@ -167,6 +169,83 @@ def test_lists_of_the_host_plan():
     cl, tp = hp.array(L.G_BASE + L.A_CHUNKLIST), hp.array(L.FEA_A_G_TILEPTR)
     assert tp[0] == 0 and tp[-1] == len(cl) and np.all(np.diff(tp) > 0) and len(tp) > 3
     assert np.all(np.diff([nodeinc[n] for n in cl[tp[:-1]]] + [nodeinc[-1]]) <= 128)
+
+
+@gpu
+@pytest.mark.parametrize("kind", [(1, 1, 1), (3, 2, 2), (9, 8, 7), "fan", "mixed"])
+def test_lists_made_on_the_device(kind):
+    """The device's lists are the host plan's: nodes of 1 to 120 elements and up
+    to 122 neighbours, partly and wholly fixed ones, nodes that also belong to
+    C3D8 elements or to no element."""
+    from fea_b200 import DevicePlan
+    from fea_b200 import _lib as L
+    from fea_b200.meshes import hex_block
+    rng = np.random.default_rng(6)
+    X, el = mesh((5, 4, 3) if kind == "mixed" else kind)
+    groups = [("C3D4", el)]
+    if kind == "mixed":
+        groups.insert(0, ("C3D8", rng.permutation(len(X))[hex_block(0, dims=(4, 3, 3))[1]]))
+        X, el = np.concatenate([X, rng.uniform(size=(3, 3))]), el[::2]
+        groups[1] = ("C3D4", el)
+    mask = rng.choice(np.array([7, 7, 7, 7, 5, 2, 0], np.uint8), len(X))
+    P = DevicePlan(X, mask, groups)
+    gi = len(groups) - 1
+    g = P.groups[gi]
+    assert g.lists is None and not g.desc.clist_dev           # (made when asked for)
+    want = [P.host.array(a, gi) for a in (L.FEA_A_G_CLIST, L.FEA_A_G_CREC)]
+    assert (want[0].size, want[1].size) == (4 * g.ninc, 2 * g.nrec)
+    out = [torch.full((w.size + 16,), -7, dtype=t, device="cuda") for w, t in zip(want, (torch.int16, torch.int32))]
+    L.check(L.fea_tet_lists(C.byref(P.nodes), C.byref(g.desc), ptr(out[0]), ptr(out[1]),
+                            C.c_void_p(torch.cuda.current_stream().cuda_stream)), "lists")
+    for w, o in zip(want, out):
+        assert np.array_equal(o[:-16].cpu().numpy().view(w.dtype), w) and bool((o[-16:] == -7).all())
+    d, _ = P.tangent_lists(gi)
+    assert d is g.desc and torch.equal(g.lists[0], out[0][:-16]) and torch.equal(g.lists[1], out[1][:-16])
+
+
+@gpu
+@pytest.mark.parametrize("first", ["capture", "stream", "threads"])
+def test_first_tangent(first):
+    """The lists come with the first tangent: under capture (whose replays make
+    their own), on another stream, from several threads at once; a later
+    tangent elsewhere has the same bits."""
+    import threading
+    from fea_b200 import DevicePlan
+    X, el = mesh((9, 8, 7))
+    P, Q = (DevicePlan(X, np.full(len(X), 7, np.uint8), [("C3D4", el)]) for _ in range(2))
+    gc = torch.from_numpy(np.random.default_rng(2).normal(0, 1e-3, P.ndof)).cuda()
+
+    def tangent(p, K):
+        p.assemble_volume(0, 1.0, 30.0, gc, K=K)
+        return K
+    ref = tangent(Q, P.zeros(P.nnz))
+    Ks = [P.zeros(P.nnz) for _ in range(4)]
+    torch.cuda.synchronize()
+    if first == "capture":
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            tangent(P, Ks[0])
+        assert P.groups[0].lists is None
+        tangent(P, Ks[1])                         # before the first replay
+        for _ in range(2):
+            Ks[0].zero_()
+            g.replay()
+    elif first == "stream":
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            tangent(P, Ks[0])
+        tangent(P, Ks[1])
+    else:
+        def go(k):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                tangent(P, Ks[k])
+                torch.cuda.current_stream().synchronize()
+        th = [threading.Thread(target=go, args=(k,)) for k in range(4)]
+        [t.start() for t in th]
+        [t.join() for t in th]
+    torch.cuda.synchronize()
+    for k in range(4 if first == "threads" else 2):
+        assert torch.equal(Ks[k], ref)
 
 
 @gpu
