@@ -471,8 +471,9 @@ extern "C" int fea_explicit_stage(int64_t n, int32_t stage, double dt, const dou
   return (int)cudaGetLastError();
 }
 
-// second u buffer (ndof doubles, rounded to 16 bytes), then the two
-// node-major copies of coordinates and u (6 doubles per node each)
+// ndof doubles (rounded to 16 bytes) that are part of the published length and
+// not used, then the two node-major copies of coordinates and u (6 doubles per
+// node each)
 extern "C" int64_t fea_explicit_work_len(const fea_nodes_t* N) {
   if (!N || N->ndof < 0 || N->n_nodes < 0) return 0;
   return ((N->ndof + 1) & ~(int64_t)1) + 12 * N->n_nodes;

@@ -231,3 +231,32 @@ def test_batched_pcg_rejects_a_bad_table_before_touching_the_device():
     assert L.fea_pcgb_state(T, 4, 1000, 2, None, None) == EINVAL
     assert L.fea_pcgb_state(T, 4, 1000, 0, None, None) == 0
     assert L.fea_launch_count() == n0
+
+
+def test_tangent_lists_check_arguments_first():
+    from fea_b200 import _lib as L
+    n0 = L.fea_launch_count()
+    N, g = _nodes(), _group(L.FEA_C3D4, 4, 256)
+
+    def lists(G=g, nodes=N, clist=_p(1), crec=_p(2)):
+        return L.fea_tet_lists(C.byref(nodes) if nodes is not None else None, C.byref(G) if G is not None else None,
+                               clist, crec, None)
+    assert lists(nodes=None) == EINVAL and lists(G=None) == EINVAL
+    assert lists(_group(L.FEA_C3D8, 8, 32)) == EINVAL
+    assert lists(clist=None) == EINVAL and lists(crec=None) == EINVAL
+    assert lists(crec=C.c_void_p(FAKE + 4)) == EINVAL               # not 8-byte aligned
+    for f in ("boff_dev", "nodeinc_dev", "crecptr_dev"):
+        h = _group(L.FEA_C3D4, 4, 256)
+        setattr(h, f, None)
+        assert lists(h) == EINVAL, f
+    for f in ("mask_dev", "adjptr_dev", "adjcol_dev", "adjoff_dev"):
+        M = _nodes()
+        setattr(M, f, None)
+        assert lists(nodes=M) == EINVAL, f
+    h = _group(L.FEA_C3D4, 4, 256)
+    h.maxval = 129                                                  # more incidences than a tile holds
+    assert lists(h) == ECHUNK
+    M = _nodes()
+    M.n_nodes = 0
+    assert lists(nodes=M) == 0
+    assert L.fea_launch_count() == n0

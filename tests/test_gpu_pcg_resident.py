@@ -72,6 +72,19 @@ def test_matches_plain_csr_pcg(kind, dims, fixed, shuffle):
     assert torch.equal(xa, xc)                         # bitwise the same from run to run
 
 
+@pytest.mark.parametrize("kind,dims,resident", [("C3D8", (1, 1, 1), True), ("C3D4", (24, 6, 5), True),
+                                                ("C3D8", (23, 22, 22), True), ("C3D8", (26, 26, 26), False)])
+def test_which_systems_are_resident(kind, dims, resident):
+    """A resident solve of 300 iterations is a few launches, the kernels per
+    part are two an iteration."""
+    from fea_b200 import _lib as L
+    P, K, b = system(kind, dims)
+    n0 = L.fea_launch_count()
+    assert P.pcg(K, b, torch.zeros_like(b), 1e-300, 300)[0] <= 300
+    n = L.fea_launch_count() - n0
+    assert n <= 20 if resident else n >= 600
+
+
 def test_caps_guesses_and_breakdown():
     from fea_b200 import _lib as L
     P, K, b = system("C3D8", (10, 9, 9))
