@@ -190,14 +190,15 @@ def test_plans_hold_no_slots(monkeypatch):
 
     def plan():
         return DevicePlan(X, np.full(len(X), 7, np.uint8), [("C3D8", el)])
+    def used():                                   # (what was asked for, not the blocks it got)
+        return torch.cuda.memory_stats()["requested_bytes.all.current"]
     P = plan()
-    torch.cuda.synchronize()
-    before = torch.cuda.memory_allocated()
+    before = used()
     Q = plan()
-    held = torch.cuda.memory_allocated() - before
+    held = used() - before
     arrays = sum(t.numel() * t.element_size() for o in (Q, Q.groups[0]) for t in vars(o).values() if isinstance(t, torch.Tensor))
     slots = 8 * 32 * len(el)
-    assert arrays <= held < arrays + slots / 4
+    assert 0.9 * arrays < held < arrays + slots / 4
     gc = 1e-3 * torch.randn(P.ndof, dtype=torch.float64, generator=torch.Generator().manual_seed(5)).cuda()
     lam = torch.randn(P.n_nodes, 3, dtype=torch.float64, generator=torch.Generator().manual_seed(4)).cuda()
     out, empty = [], torch.empty
@@ -208,13 +209,13 @@ def test_plans_hold_no_slots(monkeypatch):
         return empty(n, *a, **k)
     for tight in (True, False):
         R, dX, dmu = P.zeros(P.ndof), torch.zeros_like(lam), P.zeros(1)
-        before = torch.cuda.memory_allocated()
+        before = used()
         with monkeypatch.context() as m:
             if tight:
                 m.setattr(torch, "empty", no_room)
             P.assemble_volume(0, 1.0, 40.0, gc, R=R)
             P.adjoint_vjp_volume(0, 1.0, 40.0, gc, lam, dX, dmu)
-        assert torch.cuda.memory_allocated() - before < slots / 4
+        assert used() - before < slots / 4
         out.append((R, dX))
     assert not torch.equal(*[o[0] for o in out])  # two paths, to rounding the same
     for x, y in zip(*out):
