@@ -143,10 +143,12 @@ class GatherGroup:
         # C3D4: places of the tangent's neighbour records and its tiles (the
         # lists themselves with the first tangent, DevicePlan.tangent_lists)
         self.crecptr = self.tileptr = self.lists = None
+        self.lists_done = True
         crecptr = hp.array(L.FEA_A_G_CRECPTR, index) if base == L.G_BASE else np.zeros(0, np.int64)
         if crecptr.size and nodeinc[-1] > 0:
             self.crecptr, self.tileptr = dev(crecptr), dev(hp.array(L.FEA_A_G_TILEPTR, index))
             self.ninc, self.nrec = int(nodeinc[-1]), int(crecptr[-1])
+            self.lists_done = False
         self.allptr = dev(hp.array(base + L.A_ALLPTR, index))
         self.allinc = dev(hp.array(base + L.A_ALLINC, index))
         self.ne = int(self.conn.shape[0])
@@ -249,16 +251,21 @@ class DevicePlan:
     def tangent_lists(self, gi):
         """(descriptor, buffers) of group gi for a tangent: a C3D4 group's with
         its neighbour lists (fea_tet_lists), made on the device with the
-        group's first tangent and kept; any other group's as it is.  The
-        first caller waits for them, so that every stream may use them.  A
-        capture that comes first takes lists of its own, made anew by each
-        replay.  Without memory for them the tangent is summed in rank
+        group's first tangent and kept; any other group's as it is.  Calls on
+        other streams wait on the device until the lists are there; a capture
+        that cannot know that they are takes lists of its own, made anew by
+        each replay.  Without memory for them the tangent is summed in rank
         rounds."""
         g = self.groups[gi]
-        if g.crecptr is None or g.lists is not None:
+        if g.lists_done:
             return g.desc, None
         with self._lists_lock:
-            if g.lists is not None:
+            capturing = torch.cuda.is_current_stream_capturing()
+            if g.lists is not None and not capturing:
+                if g.lists[2].query():
+                    g.lists_done = True
+                else:
+                    torch.cuda.current_stream().wait_event(g.lists[2])
                 return g.desc, None
             try:
                 clist = torch.empty(4 * g.ninc, dtype=torch.int16, device=self.device)
@@ -266,13 +273,14 @@ class DevicePlan:
             except torch.cuda.OutOfMemoryError:
                 return g.desc, None
             L.check(L.fea_tet_lists(C.byref(self.nodes), C.byref(g.desc), vptr(clist), vptr(crec), stream()), "fea_tet_lists")
-            if torch.cuda.is_current_stream_capturing():
+            if capturing:
                 d = L.Group.from_buffer_copy(g.desc)
                 d.clist_dev, d.crec_dev = vptr(clist), vptr(crec)
                 return d, (clist, crec)
-            torch.cuda.current_stream().synchronize()
+            ready = torch.cuda.Event()
+            ready.record()
+            g.lists = (clist, crec, ready)
             g.desc.clist_dev, g.desc.crec_dev = vptr(clist), vptr(crec)
-            g.lists = (clist, crec)
         return g.desc, None
 
     def slots(self, n):
@@ -291,7 +299,7 @@ class DevicePlan:
         need(K, self.nnz, self.device, "K")
         need(R, self.ndof, self.device, "R")
         need(elemR, g.nn * 3 * g.ne, self.device, "elemR")
-        d, keep = self.tangent_lists(gi) if K is not None else (g.desc, None)
+        d, keep = (g.desc, None) if K is None or g.lists_done else self.tangent_lists(gi)
         w = self.stage(gi)[0] if K is not None else self.slots(g.force_len) if g.once else None
         L.check(L.fea_assemble_volume(C.byref(self.nodes), C.byref(d), float(mu), float(kappa), vptr(gc),
                                       vptr(K), vptr(R), vptr(elemR), int(bool(accumulate)), vptr(w),

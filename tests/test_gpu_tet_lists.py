@@ -204,11 +204,11 @@ def test_lists_made_on_the_device(kind):
 
 
 @gpu
-@pytest.mark.parametrize("first", ["capture", "stream", "threads"])
+@pytest.mark.parametrize("first", ["capture", "warm", "stream", "threads"])
 def test_first_tangent(first):
     """The lists come with the first tangent: under capture (whose replays make
-    their own), on another stream, from several threads at once; a later
-    tangent elsewhere has the same bits."""
+    their own), before one, on another stream, from several threads at once; a
+    later tangent elsewhere has the same bits."""
     import threading
     from fea_b200 import DevicePlan
     X, el = mesh((9, 8, 7))
@@ -230,6 +230,15 @@ def test_first_tangent(first):
         for _ in range(2):
             Ks[0].zero_()
             g.replay()
+    elif first == "warm":
+        tangent(P, Ks[1])
+        torch.cuda.synchronize()
+        tangent(P, Ks[1])
+        assert P.groups[0].lists_done             # the capture takes the plan's lists
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            tangent(P, Ks[0])
+        g.replay()
     elif first == "stream":
         s = torch.cuda.Stream()
         with torch.cuda.stream(s):
