@@ -114,3 +114,26 @@ def test_search_direction_has_the_same_bits_at_every_size(copies):
     one, many = solve(1), solve(copies)
     assert float((one != 0).double().mean()) > 0.99
     assert float((many != one).double().mean()) < 1e-5
+
+
+@pytest.mark.parametrize("dims,rows", [((26, 26, 26), 56862), ((27, 27, 27), 63504)])
+def test_plan_layout_solve_on_both_sides_of_the_pairs_line(dims, rows):
+    """FP32 values in the plan's layout below and above the 60,000 rows from
+    which p has an array of its own, against the FP64 solve: both meet the FP64
+    stop test at 1e-16 (squared), and the iterates differ by sqrt(cond) of its
+    root, below 1e-5 of the largest entry."""
+    from fea_b200 import DevicePlan
+    from fea_b200.meshes import hex_block
+    X, el = hex_block(0, dims=dims)
+    mask = np.full(len(X), 7, np.uint8)
+    mask[X[:, 0] == 0] = 0
+    P = DevicePlan(X, mask, [("C3D8", el)])
+    assert P.ndof == rows
+    K = P.zeros(P.nnz)
+    P.assemble_volume(0, 1.0, 10.0, P.zeros(P.ndof), K=K)
+    b = torch.from_numpy(np.random.default_rng(1).normal(size=P.ndof)).cuda()
+    x, y = torch.zeros_like(b), torch.zeros_like(b)
+    it, out, rr, st = P.pcg_mixed(K, P.to_f32(K), b, x, 1e-16, 0.0, 20000, check_every=50)
+    assert st == 0 and out >= 1 and rr < 1e-16
+    assert P.pcg(K, b, y, 1e-22, 20000)[2] == 0
+    assert float((x - y).abs().max()) <= 1e-5 * float(y.abs().max())
